@@ -18,7 +18,7 @@
  *     refinement sweep, gpu_kin_set_mixed_variant)
  *   - gpu_kin_advance_queue: persistent kernel over a device work queue
  *   - gpu_kin_autotune / gpu_kin_get_tuning: launch-shape autotuner
- *   - gpu_kin_set_straggler_budget: FP64 straggler hand-off to the cooperative kernel
+ *   - gpu_kin_set_straggler_budget: FP64 straggler hand-off to the group kernels
  *   - gpu_kin_coop_*: cooperative (one CTA per cell) kernels for large mechanisms
  *   - gpu_advect, gpu_serve_*: film advection, CUDA-graph coupling step, serving
  *   - kin_model_*: host-side mechanism compiler (the reference's kin_build.cpp)
@@ -180,7 +180,8 @@ SGB_API int32_t gpu_kin_advance_async(const GpuKinLaunch *launch, void *host_blo
                                       uint64_t mutable_rows);
 /* gpu_api.h:105 */
 SGB_API int32_t gpu_kin_wait(float *kernel_ms, float *total_ms);
-/* gpu_api.h:109 -- 0 = one thread per cell, 1 = one warp per cell (FP64 and mixed advances run the
+/* gpu_api.h:109 -- 0 = by size (one thread per cell for batches that fill the GPU, 8 to 32 lanes per cell
+ * for smaller ones; the same bits), 1 = one warp per cell (FP64 and mixed advances run the
  * cooperative kernel with 32 threads per cell; FP64 keeps the same bits). */
 SGB_API int32_t gpu_kin_set_mode(uint32_t mode);
 
@@ -211,7 +212,8 @@ SGB_API int32_t gpu_kin_advance_pipelined(const GpuKinLaunch *launch, void *host
  * as fit), variant = compiled register-budget variant (0: up to 255 registers
  * at 128 threads, 1: 128 registers, 2: 255 registers at 256 threads, kind 2
  * only; 3: 128 registers at 512 threads, kind 2 only); for kind 3, chunk =
- * CTAs per SM (1..8, 0 = 8).
+ * CTAs per SM (1..8, 0 = 8). Until one is set or measured, the module chooses by batch
+ * size, lane-group kernels (8, 16 or 32 lanes per cell; the same bits) included.
  * gpu_kin_autotune times the candidates of `kind` on the given launch (which
  * it advances repeatedly on a scratch copy it restores) and keeps the fastest;
  * kind 4 times kinds 2 and 3 together, so the cells-per-warp decomposition is
@@ -235,16 +237,16 @@ SGB_API int32_t gpu_kin_set_refinement(uint32_t sweeps);
  * (only the scalar step controller stays FP64). Default 1. */
 SGB_API int32_t gpu_kin_set_mixed_variant(uint32_t variant);
 /* Straggler hand-off for precision 0 (0 = off; default 600): in one advance, a cell still
- * stepping after `attempts` step attempts on its lane is parked and finished right after by the
- * FP64 cooperative kernel (one CTA per cell, every thread sharing the cell's work), so a few very
- * stiff cells no longer run alone on single lanes at the end of the launch; the results keep
- * the same bits. The mixed path does not hand off: its lanes' FP32-pipe steps are shorter
- * than the cooperative FP64 steps. */
+ * stepping after `attempts` step attempts on its lane is parked and finished right after by a
+ * group kernel (a warp per cell), so a few very stiff cells no longer run alone on single lanes
+ * at the end of the launch; the results keep the same bits. The mixed lane kernels keep their
+ * cells. */
 SGB_API int32_t gpu_kin_set_straggler_budget(uint32_t attempts);
 /* Per-thread stack (local memory) reservation of the current context: set it when set_bytes
  * is nonzero; *current receives the value in force. */
 SGB_API int32_t gpu_stack_limit(uint64_t set_bytes, uint64_t *current);
-/* Threads of the cooperative kernel per parked cell (32..256, multiple of 32; default 128). */
+/* Kept for callers (32..256, multiple of 32): parked cells run on the group kernels, which choose their
+ * own shape. */
 SGB_API int32_t gpu_kin_set_straggler_block(uint32_t threads);
 /* Cells parked by the last advance that used the hand-off (waits for the module stream). */
 SGB_API int32_t gpu_kin_parked_cells(uint32_t *count);
@@ -515,6 +517,10 @@ SGB_API uint64_t kin_mech_signature(const KinMech *mech); /* FNV-1a over the rec
  * `out` when `capacity` suffices. The same mechanism gives the same bytes from either source. */
 SGB_API uint64_t kin_model_coop_image(const KinModelHandle *model, void *out, uint64_t capacity);
 SGB_API uint64_t kin_mech_coop_image(const KinMech *mech, void *out, uint64_t capacity);
+/* The lane-group kernels' schedule image of a KinMech for 8, 16 or 32 lanes per cell and a lane precision
+ * (0 FP64, 1 f32 Delta, 4 mixed): its size, 0 if the record is not what the symbolic phase makes
+ * (the lane kernels then run alone); copied to `out` when `capacity` suffices. */
+SGB_API uint64_t kin_mech_group_image(const KinMech *mech, uint32_t lanes, uint32_t lane_precision, void *out, uint64_t capacity);
 SGB_API void kin_model_rate_constants(const KinModelHandle *model, double T, double M, double *k);
 /* Rate constants for `cells` cells of a [reactions][padded] block from T and M per cell. */
 SGB_API void kin_model_rate_block(const KinModelHandle *model, const double *T, const double *M, uint32_t cells,

@@ -218,6 +218,7 @@ def lib() -> C.CDLL:
             "kin_mech_signature": (u64, [C.POINTER(KinMech)]),
             "kin_model_coop_image": (u64, [vp, vp, u64]),
             "kin_mech_coop_image": (u64, [C.POINTER(KinMech), vp, u64]),
+            "kin_mech_group_image": (u64, [C.POINTER(KinMech), u32, u32, vp, u64]),
             "kin_model_rate_constants": (None, [vp, d, d, vp]),
             "kin_model_rate_block": (None, [vp, vp, vp, u32, u32, vp]),
             "kin_method_coefficients": (KinMethod, [u32]),
@@ -553,7 +554,7 @@ class Module:
         return int(lib().gpu_kin_get_mixed_variant())
 
     def set_straggler_budget(self, attempts: int) -> None:
-        """Cells still stepping after `attempts` attempts are finished by the cooperative kernel (0 = off)."""
+        """Cells still stepping after `attempts` attempts are finished by a group kernel (0 = off)."""
         check(lib().gpu_kin_set_straggler_budget(attempts), "gpu_kin_set_straggler_budget")
 
     def parked_cells(self) -> int:

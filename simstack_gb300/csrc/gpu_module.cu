@@ -16,6 +16,7 @@
 #include "mech.h"
 #include "mech_tables.h"
 #include "coop.h"
+#include "group.h"
 
 #include <vector>
 
@@ -79,6 +80,8 @@ struct Module {
     uint32_t *d_error = nullptr;   // bounded-wait error flag
     uint32_t mode = 0;
     GpuKinTuning tuning[3];
+    bool tuned[3] = {};            // the caller set or measured this precision's tuning: it runs as it is
+    GroupSet group;                // schedule images of the lane-group kernels (none: lane kernels only)
     uint32_t ir_sweeps = 1;
     uint32_t wait_polls = kSpinLimit;   // poll limit of the table-staging waits
     // precision 2: 0 FP64-residual refinement, 1 double-float state, 2 double-float state with
@@ -92,12 +95,13 @@ struct Module {
     cudaEvent_t ev_in[kMaxChunks] = {}, ev_kern[kMaxChunks] = {};
     cudaEvent_t pipe_begin = nullptr, pipe_end = nullptr, pipe_after = nullptr;
     // straggler hand-off: cells past `straggler_budget` step attempts in one launch are parked
-    // and finished by the cooperative kernel (one CTA per cell) on the same stream
+    // and finished by a group kernel on the same stream
     uint32_t straggler_budget = 600;  // FP64 step attempts per launch before a cell is handed on
-    uint32_t straggler_block = 128;   // threads per parked cell
     SuspendRec *d_suspend = nullptr;
     uint32_t *d_suspend_count = nullptr;
-    void *d_coop_image = nullptr;
+    void *d_coop_image = nullptr;     // coop_image_buffer while the mechanism has an image
+    void *coop_image_buffer = nullptr;
+    size_t coop_image_bytes = 0, coop_scratch_bytes = 0;
     CoopMech coop_head;
     double *d_coop_scratch = nullptr;
     uint32_t coop_grid = 0;
@@ -112,7 +116,7 @@ constexpr uint32_t kSuspendCap = 1u << 16;       // parked cells per launch
 // different reservations and reallocations); 3,840 bytes covers every default-path kernel of
 // the shipped mechanism (the FP64 lanes need 3,680) and was the fastest such size measured.
 constexpr size_t kStackReserveBytes = 3840;
-constexpr uint32_t kResumeCtasPerSm = 8;         // cooperative CTAs per SM for parked cells
+constexpr uint32_t kCoopCtasPerSm = 8;           // cooperative CTAs per SM at most (tuning kind 3)
 
 
 const GpuKinTuning kDefaultTuning = {2u, 128u, 0u, 0u, 0.0f};   // CTA-synchronous queue, 128 threads, 255 registers
@@ -161,6 +165,42 @@ cudaError_t occupancy(uint32_t prec, const GpuKinTuning &t, int *blocks) {
 
 cudaError_t launch_lanes(uint32_t prec, const GpuKinTuning &t, const DevArgs &A, cudaStream_t stream = nullptr);
 
+GpuKinTuning tuning_for(uint32_t p);
+
+// The lane type a precision runs (LaneOf, kin_kernels.cuh).
+uint32_t lane_prec(uint32_t prec) { return prec == 2 ? 2u + g.mixed_variant : prec; }
+
+// Launch shape of an advance: a group kernel (group >= 0: kGroupLanes[group] lanes per cell) or the lane
+// kernels at `t`.
+struct AdvanceShape {
+    int group;
+    GpuKinTuning t;
+};
+
+// The shape of an advance of `lanes` cells: the caller's tuning where one was set or measured,
+// else by size. A lane kernel takes as long for one cell per SM as for a full warp of them (shipped
+// mechanism, 1 s: FP64 59 ms, mixed 25 ms up to 16,384 cells), so small batches go to the group
+// kernels (group_rule in group.h).
+AdvanceShape shape_for(uint32_t prec, uint32_t lanes, bool with_mode) {
+    AdvanceShape s = {-1, with_mode ? tuning_for(prec) : g.tuning[prec]};
+    if (g.tuned[prec] || (with_mode && g.mode == 1) || s.t.kind == 3 || !g.group.dev) return s;
+    s.group = group_rule(lane_prec(prec), g.generated, lanes, g.sms);
+    return s;
+}
+
+// Whether a lane advance of this precision hands its stragglers on.
+bool handoff(uint32_t prec) { return g.straggler_budget && g.group.dev && prec == 0; }
+
+// The group kernel on cells of `A` (its cursor is zeroed first), or on the parked ones (A.resume).
+cudaError_t launch_group(uint32_t prec, int group, const DevArgs &A0, cudaStream_t stream) {
+    DevArgs A = A0;
+    A.budget = g.straggler_budget;
+    if (g.generated) A.wait_polls = kSpinLimit;   // the caller's limit is for a table mechanism's staging
+    cudaError_t e = cudaMemsetAsync(A.cursor, 0, sizeof(uint32_t), stream);
+    if (e != cudaSuccess) return e;
+    return g.group.launch(lane_prec(prec), group, A, A.resume ? kSuspendCap : A.lanes, g.sms, stream);
+}
+
 // Local memory per thread the kernel of (precision, tuning) needs.
 cudaError_t local_bytes(uint32_t prec, const GpuKinTuning &t, size_t *bytes) {
     if (t.kind == 3) {   // the cooperative kernel keeps its state in shared and global memory
@@ -178,29 +218,26 @@ cudaError_t local_bytes(uint32_t prec, const GpuKinTuning &t, size_t *bytes) {
     return prec == 0 ? local_table_p0(t.kind, bytes) : prec == 1 ? local_table_p1(t.kind, bytes) : local_table_p2(t.kind, bytes);
 }
 
-// Launches one advance of `A` with tuning `t` on the module stream; with a
-// straggler budget (precision 0), cells still stepping after that many
-// attempts are parked and finished by the FP64 cooperative kernel right after,
-// with the same bits. (The mixed lanes' FP32-pipe steps are shorter than the
-// cooperative FP64 steps, so they keep their cells.)
-cudaError_t launch_advance(uint32_t prec, const GpuKinTuning &t, const DevArgs &A0) {
+// Launches one advance of `A` in shape `s` on the module stream; the lane kernels with a straggler
+// budget (precision 0) park cells still stepping after that many attempts, and a group kernel
+// finishes them right after, with the same bits.
+cudaError_t launch_advance(uint32_t prec, const AdvanceShape &s, const DevArgs &A0) {
     if (A0.lanes == 0) return cudaSuccess;
+    if (s.group >= 0) return launch_group(prec, s.group, A0, g.stream);
+    const GpuKinTuning &t = s.t;
     if (t.kind == 3) {   // cooperative decomposition: one cell per CTA of t.block threads (32: one warp per cell)
         if (!g.d_coop_image || prec == 1) return cudaErrorInvalidValue;
         DevArgs R = A0;
-        R.budget = 0;
-        R.resume = 0;
         R.tables = g.d_coop_image;
         R.table_bytes = g.coop_head.bytes;
-        const uint32_t per_sm = t.chunk ? (t.chunk < kResumeCtasPerSm ? t.chunk : kResumeCtasPerSm) : kResumeCtasPerSm;
+        const uint32_t per_sm = t.chunk ? (t.chunk < kCoopCtasPerSm ? t.chunk : kCoopCtasPerSm) : kCoopCtasPerSm;
         uint32_t grid = (uint32_t)g.sms * per_sm;
         if (grid > A0.lanes) grid = A0.lanes;
         cudaError_t e = cudaMemsetAsync(A0.cursor, 0, sizeof(uint32_t), g.stream);
         if (e != cudaSuccess) return e;
         return coop_launch((int)prec, R, g.coop_head, g.d_coop_scratch, grid, t.block, g.stream);
     }
-    const bool handoff = g.straggler_budget && g.d_coop_image && prec == 0;
-    if (!handoff) return launch_lanes(prec, t, A0);
+    if (!handoff(prec)) return launch_lanes(prec, t, A0);
     DevArgs A = A0;
     A.budget = g.straggler_budget;
     A.suspend_cap = kSuspendCap;
@@ -209,14 +246,9 @@ cudaError_t launch_advance(uint32_t prec, const GpuKinTuning &t, const DevArgs &
     cudaError_t e = cudaMemsetAsync(g.d_suspend_count, 0, sizeof(uint32_t), g.stream);
     if (e == cudaSuccess) e = launch_lanes(prec, t, A);
     if (e != cudaSuccess) return e;
-    DevArgs R = A;
-    R.budget = 0;
-    R.resume = 1;
-    R.tables = g.d_coop_image;
-    R.table_bytes = g.coop_head.bytes;
-    e = cudaMemsetAsync(g.d_cursor, 0, sizeof(uint32_t), g.stream);
-    if (e != cudaSuccess) return e;
-    return coop_launch(0, R, g.coop_head, g.d_coop_scratch, g.coop_grid, g.straggler_block, g.stream);
+    A.resume = 1;
+    A.cursor = g.d_cursor;
+    return launch_group(prec, 0, A, g.stream);
 }
 
 // The lane kernels (one cell per thread) for `A`, on `stream` (default: the module stream); the
@@ -289,14 +321,14 @@ cudaError_t read_error_flag() {
     return cudaSuccess;
 }
 
-// Timed advance on the module stream; waits for completion.
-cudaError_t advance_sync(const GpuKinLaunch *L, const GpuKinTuning &t, float *kernel_ms) {
+// Timed advance on the module stream at `t` (null: shape_for's choice); waits for completion.
+cudaError_t advance_sync(const GpuKinLaunch *L, const GpuKinTuning *t, float *kernel_ms) {
     cudaError_t e = check_launch(L);
     if (e != cudaSuccess) return e;
     DevArgs A;
     fill_args(L, &A);
     cudaEventRecord(g.kin_start, g.stream);
-    e = launch_advance(L->precision, t, A);
+    e = launch_advance(L->precision, t ? AdvanceShape{-1, *t} : shape_for(L->precision, A.lanes, true), A);
     cudaEventRecord(g.kin_stop, g.stream);
     if (e != cudaSuccess) return e;
     e = cudaEventSynchronize(g.kin_stop);
@@ -380,7 +412,10 @@ SGB_API int32_t gpu_init(uint32_t device_index, uint64_t arena_bytes, GpuInfo *i
     }
     g.device = (int)device_index;
     g.sms = prop.multiProcessorCount;
-    for (int p = 0; p < 3; ++p) g.tuning[p] = kDefaultTuning;
+    for (int p = 0; p < 3; ++p) {
+        g.tuning[p] = kDefaultTuning;
+        g.tuned[p] = false;
+    }
     g.have_mech = false;
     g.ready = true;
     return (int32_t)cudaGetLastError();
@@ -457,6 +492,19 @@ SGB_API int32_t gpu_step_points(float *x, float *y, float *z, float *vx, float *
     return (int32_t)cudaGetLastError();
 }
 
+namespace {
+// A device buffer of at least `bytes`: kept, or replaced by a larger one.
+cudaError_t grow(void **buffer, size_t *have, size_t bytes) {
+    if (*have >= bytes) return cudaSuccess;
+    if (*buffer) cudaFree(*buffer);
+    *buffer = nullptr;
+    *have = 0;
+    const cudaError_t e = cudaMalloc(buffer, bytes);
+    if (e == cudaSuccess) *have = bytes;
+    return e;
+}
+}   // namespace
+
 SGB_API int32_t gpu_kin_set_mech(const KinMech *mech, const KinMethod *method, const KinControl *control) {
     if (!g.ready) return (int32_t)cudaErrorInitializationError;
     if (!mech || !method || !control) return (int32_t)cudaErrorInvalidValue;
@@ -472,24 +520,21 @@ SGB_API int32_t gpu_kin_set_mech(const KinMech *mech, const KinMethod *method, c
     g.control = *control;
     g.generated = fnv1a(mech, sizeof(KinMech)) == air_ops_signature() && method_is_rodas3(method);
     g.have_mech = true;
-    // the cooperative image of the same mechanism, for the straggler hand-off (none: no hand-off)
-    if (g.d_coop_image) cudaFree(g.d_coop_image);
-    if (g.d_coop_scratch) cudaFree(g.d_coop_scratch);
+    e = g.group.build(*mech, method_is_rodas3(method));
+    if (e != cudaSuccess) return (int32_t)e;
+    // the cooperative image of the same mechanism (tuning kind 3, mode 1)
+    // (the buffers are kept while they are large enough: the stream is idle here)
     g.d_coop_image = nullptr;
-    g.d_coop_scratch = nullptr;
     std::vector<uint8_t> coop;
     if (coop_image(*mech, &coop)) {
         memcpy(&g.coop_head, coop.data(), sizeof(CoopMech));
-        g.coop_grid = (uint32_t)g.sms * kResumeCtasPerSm;
+        g.coop_grid = (uint32_t)g.sms * kCoopCtasPerSm;
         const size_t a = coop_scratch_doubles_for(0, g.coop_head), b = coop_scratch_doubles_for(2, g.coop_head);
-        e = cudaMalloc(&g.d_coop_image, coop.size());
-        if (e == cudaSuccess) e = cudaMemcpy(g.d_coop_image, coop.data(), coop.size(), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMalloc((void **)&g.d_coop_scratch, (a > b ? a : b) * 8 * g.coop_grid);
-        if (e != cudaSuccess) {
-            if (g.d_coop_image) cudaFree(g.d_coop_image);
-            g.d_coop_image = nullptr;
-            return (int32_t)e;
-        }
+        e = grow(&g.coop_image_buffer, &g.coop_image_bytes, coop.size());
+        if (e == cudaSuccess) e = cudaMemcpy(g.coop_image_buffer, coop.data(), coop.size(), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = grow((void **)&g.d_coop_scratch, &g.coop_scratch_bytes, (a > b ? a : b) * 8 * g.coop_grid);
+        if (e != cudaSuccess) return (int32_t)e;
+        g.d_coop_image = g.coop_image_buffer;
     }
     return 0;
 }
@@ -497,6 +542,7 @@ SGB_API int32_t gpu_kin_set_mech(const KinMech *mech, const KinMethod *method, c
 // The tuning an advance of precision p runs: mode 1 (the reference's warp per cell) is the
 // cooperative decomposition with one warp per cell for FP64 and mixed; f32 lanes keep one thread
 // per cell in either mode.
+namespace {
 GpuKinTuning tuning_for(uint32_t p) {
     GpuKinTuning t = g.tuning[p];
     if (g.mode == 1 && p != 1 && t.kind != 3) {
@@ -506,11 +552,12 @@ GpuKinTuning tuning_for(uint32_t p) {
     }
     return t;
 }
+}   // namespace
 
 SGB_API int32_t gpu_kin_advance(const GpuKinLaunch *launch, float *kernel_ms) {
     uint32_t p = launch ? launch->precision : 0;
     if (p > 2) return (int32_t)cudaErrorInvalidValue;
-    return (int32_t)advance_sync(launch, tuning_for(p), kernel_ms);
+    return (int32_t)advance_sync(launch, nullptr, kernel_ms);
 }
 
 SGB_API int32_t gpu_host_register(void *host, uint64_t size) {
@@ -540,7 +587,7 @@ SGB_API int32_t gpu_kin_advance_async(const GpuKinLaunch *launch, void *host_blo
     DevArgs A;
     fill_args(launch, &A);
     cudaEventRecord(g.kin_start, g.stream);
-    e = launch_advance(launch->precision, tuning_for(launch->precision), A);
+    e = launch_advance(launch->precision, shape_for(launch->precision, A.lanes, true), A);
     cudaEventRecord(g.kin_stop, g.stream);
     if (e != cudaSuccess) return (int32_t)e;
     e = cudaMemcpy2DAsync(host_block, pitch, device_block, pitch, width, mutable_rows, cudaMemcpyDeviceToHost, g.stream);
@@ -576,7 +623,7 @@ SGB_API int32_t gpu_kin_advance_pipelined(const GpuKinLaunch *launch, void *host
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&g.kern2, cudaStreamNonBlocking);
         if (e != cudaSuccess) return (int32_t)e;
     }
-    const bool serial = g.straggler_budget && g.d_coop_image && launch->precision == 0;
+    const bool serial = handoff(launch->precision);
     const uint64_t P = launch->padded, lanes = launch->lane_count ? launch->lane_count : launch->padded;
     const uint64_t pitch = P * sizeof(double);
     const uint64_t per = (lanes + chunks - 1) / chunks;
@@ -601,11 +648,13 @@ SGB_API int32_t gpu_kin_advance_pipelined(const GpuKinLaunch *launch, void *host
         Lc.lane_count = (uint32_t)count;
         DevArgs A;
         fill_args(&Lc, &A);
+        const AdvanceShape shape = shape_for(launch->precision, A.lanes, false);
         if (serial) {
-            e = launch_advance(launch->precision, g.tuning[launch->precision], A);
+            e = launch_advance(launch->precision, shape, A);
         } else {
             A.cursor = (uint32_t *)((uint8_t *)g.d_cursor + 256 + (size_t)c * 128);
-            e = launch_lanes(launch->precision, g.tuning[launch->precision], A, ks);
+            e = shape.group >= 0 ? launch_group(launch->precision, shape.group, A, ks)
+                                 : launch_lanes(launch->precision, shape.t, A, ks);
         }
         if (e == cudaSuccess) e = cudaEventRecord(g.ev_kern[c], ks);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(g.copy_out, g.ev_kern[c], 0);
@@ -662,19 +711,25 @@ SGB_API int32_t gpu_kin_advance_queue(const GpuKinLaunch *launch, float *kernel_
         t.variant = 0;
         t.chunk = 0;
     }
-    return (int32_t)advance_sync(launch, t, kernel_ms);
+    return (int32_t)advance_sync(launch, &t, kernel_ms);
 }
 
 SGB_API int32_t gpu_kin_set_tuning(const GpuKinTuning *t) {
     if (!t || t->kind > 3 || t->block == 0 || (t->block & 31) || t->variant > 3 || t->chunk > 64) return (int32_t)cudaErrorInvalidValue;
     if (t->kind == 3) {   // cooperative: 32..256 threads per cell
         if (t->block > 256) return (int32_t)cudaErrorInvalidValue;
-        for (int p = 0; p < 3; ++p) g.tuning[p] = *t;
+        for (int p = 0; p < 3; ++p) {
+            g.tuning[p] = *t;
+            g.tuned[p] = true;
+        }
         return 0;
     }
     const uint32_t max_block = t->variant == 3 ? 512u : t->variant == 2 ? 256u : 128u;   // the variant's __launch_bounds__
     if (t->block > max_block || (t->variant >= 2 && t->kind != 2)) return (int32_t)cudaErrorInvalidValue;
-    for (int p = 0; p < 3; ++p) g.tuning[p] = *t;
+    for (int p = 0; p < 3; ++p) {
+        g.tuning[p] = *t;
+        g.tuned[p] = true;
+    }
     return 0;
 }
 
@@ -740,7 +795,7 @@ SGB_API int32_t gpu_kin_autotune(const GpuKinLaunch *launch, uint32_t kind, GpuK
         if (keep_reservation && local_bytes(launch->precision, t, &need) == cudaSuccess && need > have) continue;
         float ms = 0.0f, best_ms = 1e30f;
         for (int rep = 0; rep < 2 && e == cudaSuccess; ++rep) {   // the faster of two runs
-            e = advance_sync(launch, t, &ms);
+            e = advance_sync(launch, &t, &ms);
             copy_all(false);
             if (ms < best_ms) best_ms = ms;
         }
@@ -754,6 +809,7 @@ SGB_API int32_t gpu_kin_autotune(const GpuKinLaunch *launch, uint32_t kind, GpuK
     cudaFree(save);
     if (e != cudaSuccess) return (int32_t)e;
     g.tuning[launch->precision] = winner;
+    g.tuned[launch->precision] = true;
     if (best) *best = winner;
     return 0;
 }
@@ -789,8 +845,7 @@ SGB_API int32_t gpu_kin_set_straggler_budget(uint32_t attempts) {
 
 SGB_API int32_t gpu_kin_set_straggler_block(uint32_t threads) {
     if (threads < 32 || threads > 256 || (threads & 31)) return (int32_t)cudaErrorInvalidValue;
-    g.straggler_block = threads;
-    return 0;
+    return 0;   // parked cells run on the group kernels, which choose their own shape
 }
 
 SGB_API int32_t gpu_kin_parked_cells(uint32_t *count) {
@@ -813,6 +868,16 @@ SGB_API int32_t gpu_kin_set_wait_limit(uint32_t polls) {
     return 0;
 }
 
+// The lane-group kernels' schedule image of a mechanism (group_tab.h).
+SGB_API uint64_t kin_mech_group_image(const KinMech *mech, uint32_t lanes, uint32_t lane_precision, void *out, uint64_t capacity) {
+    const KinMethod rodas3 = method_coefficients(2);
+    std::vector<uint32_t> img;
+    if (!mech || (lanes != 8 && lanes != 16 && lanes != 32) || (lane_precision > 1 && lane_precision != 4)) return 0;
+    if (!mech_tables_valid(mech, &rodas3) || !group_image(*mech, lanes, lane_precision, &img)) return 0;
+    if (out && capacity >= img.size() * 4) memcpy(out, img.data(), img.size() * 4);
+    return img.size() * 4;
+}
+
 namespace sgb {
 // Module settings read by the allocation-free advance (which needs no gpu_init).
 uint32_t module_wait_polls() { return g.wait_polls; }
@@ -826,7 +891,7 @@ cudaError_t module_enqueue_advance(const GpuKinLaunch *L) {
     if (e != cudaSuccess) return e;
     DevArgs A;
     fill_args(L, &A);
-    return launch_advance(L->precision, g.tuning[L->precision], A);
+    return launch_advance(L->precision, shape_for(L->precision, A.lanes, false), A);
 }
 cudaError_t module_mark_start() {
     if (!g.ready) return cudaErrorInitializationError;

@@ -1,0 +1,131 @@
+// Host side of the lane-group kernels: the device images of one mechanism and the launch.
+#pragma once
+#include <cuda_runtime.h>
+#include <string.h>
+
+#include "group_tab.h"
+#include "kin_group.cuh"
+
+namespace sgb {
+
+typedef void (*GroupFn)(DevArgs, GroupArgs);
+// The kernel of a lane precision for mechanisms of at most NM species (kern_group.cu).
+template <int PREC, int NM> GroupFn group_kernel(uint32_t G, bool rodas3);
+template <> GroupFn group_kernel<0, 12>(uint32_t, bool);
+template <> GroupFn group_kernel<0, 20>(uint32_t, bool);
+template <> GroupFn group_kernel<0, 32>(uint32_t, bool);
+template <> GroupFn group_kernel<1, 12>(uint32_t, bool);
+template <> GroupFn group_kernel<1, 20>(uint32_t, bool);
+template <> GroupFn group_kernel<1, 32>(uint32_t, bool);
+template <> GroupFn group_kernel<4, 12>(uint32_t, bool);
+template <> GroupFn group_kernel<4, 20>(uint32_t, bool);
+template <> GroupFn group_kernel<4, 32>(uint32_t, bool);
+template <int PREC> GroupFn group_kernel_for(uint32_t n, uint32_t G, bool rodas3) {
+    return n <= 12 ? group_kernel<PREC, 12>(G, rodas3) : n <= 20 ? group_kernel<PREC, 20>(G, rodas3) : group_kernel<PREC, 32>(G, rodas3);
+}
+
+// Lanes per cell of the three images.
+constexpr uint32_t kGroupLanes[3] = {8, 16, 32};
+
+// The group shape (index into kGroupLanes) for a batch of `lanes` cells on `sms` SMs, or -1: the lane
+// kernels. Lines in cells per SM, from one advance of 1 s (GB300, 152 SMs; ms for 32 / 16 / 8
+// lanes per cell and the lane kernel):
+//   shipped mechanism  600 cells: FP64 14.0 / 15.4 / 19.6 / 59.4   mixed  9.8 / 10.7 / 14.1 / 24.2
+//                    2,048 cells: FP64 20.9 / 16.7 / 20.1 / 59.4   mixed 12.2 / 11.0 / 14.4 / 25.3
+//                    4,096 cells: FP64 34.2 / 25.8 / 23.2 / 59.5   mixed 18.6 / 16.5 / 16.2 / 25.4
+//                    8,192 cells: FP64 62.7 / 44.3 / 35.4 / 59.4   mixed 33.0 / 26.5 / 23.9 / 24.8
+//                   16,384 cells: FP64  -  /  -  / 57.9 / 59.7     mixed  -  /  -  / 37.3 / 24.4
+//   24 species / 80 reactions, 1,501 cells: FP64 21.4 / 26.3 / 25.3 / 378   mixed 16.7 / 13.1 / 22.3 / 485
+// (the table-driven lane kernels keep a cell's arrays in local memory: ~1 ms per attempt).
+inline int group_rule(uint32_t lane_prec, bool generated, uint32_t lanes, int sms) {
+    const uint32_t c = (lanes + (uint32_t)sms - 1) / (uint32_t)sms;
+    if (lane_prec != 0 && lane_prec != 1 && lane_prec != 4) return -1;   // the other mixed variants: lanes only
+    if (c <= (lane_prec == 4 ? 10u : 8u)) return 2;
+    if (generated && lane_prec == 1) return c <= 12u ? 1 : -1;
+    if (c <= (lane_prec == 4 ? 26u : 16u)) return 1;
+    return c <= (!generated ? 128u : lane_prec == 4 ? 48u : 96u) ? 0 : -1;
+}
+
+// One mechanism's schedule images on the device: per lanes-per-cell and lane precision (0 FP64, 1 f32
+// Delta, 2 mixed). Empty (dev null) for a mechanism whose record could not be laid out.
+struct GroupSet {
+    unsigned char *dev = nullptr;   // set while there are images
+    unsigned char *buffer = nullptr;
+    size_t capacity = 0;
+    uint32_t offset[3][3] = {};
+    GroupHead head[3][3] = {};
+    bool rodas3 = false;
+
+    // No kernel may be using the images of the mechanism before.
+    cudaError_t build(const KinMech &mech, bool method_rodas3) {
+        dev = nullptr;
+        std::vector<uint32_t> all, one;
+        for (int g = 0; g < 3; ++g)
+            for (int f = 0; f < 3; ++f) {
+                if (!group_image(mech, kGroupLanes[g], f == 2 ? 4u : (uint32_t)f, &one)) return cudaSuccess;
+                memcpy(&head[g][f], one.data(), sizeof(GroupHead));
+                offset[g][f] = (uint32_t)all.size() * 4u;
+                all.insert(all.end(), one.begin(), one.end());
+            }
+        rodas3 = method_rodas3;
+        cudaError_t e = cudaSuccess;
+        if (all.size() * 4 > capacity) {
+            release();
+            e = cudaMalloc((void **)&buffer, all.size() * 4);
+            if (e != cudaSuccess) return e;
+            capacity = all.size() * 4;
+        }
+        e = cudaMemcpy(buffer, all.data(), all.size() * 4, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) dev = buffer;
+        return e;
+    }
+    void release() {
+        if (buffer) cudaFree(buffer);
+        dev = buffer = nullptr;
+        capacity = 0;
+    }
+
+    static int index(uint32_t lane_prec) { return lane_prec == 4 ? 2 : (int)lane_prec; }
+
+    // The kernel's arguments for G = kGroupLanes[g], and the shared memory of a CTA of `warps` warps.
+    GroupArgs args(uint32_t lane_prec, int g) const {
+        const int f = index(lane_prec);
+        GroupArgs a;
+        a.image = dev + offset[g][f];
+        a.image32 = dev + offset[2][f];
+        a.bytes = head[g][f].words * 4;
+        a.bytes32 = head[2][f].words * 4;
+        a.cell_bytes = group_cell_bytes(head[g][f], lane_prec, kGroupLanes[g]);
+        const uint32_t cells = 32u / kGroupLanes[g] * a.cell_bytes, one = group_cell_bytes(head[2][f], lane_prec, 32);
+        a.warp_bytes = kGroupStateBytes + (cells > one ? cells : one);
+        return a;
+    }
+    static size_t smem(const GroupArgs &a, int g, uint32_t warps) {
+        return (size_t)a.bytes + (g < 2 ? a.bytes32 : 0u) + (size_t)warps * a.warp_bytes;
+    }
+
+    // Enqueues the kernel on cells of `A` (A.cursor zeroed by the caller; A.resume: the parked
+    // ones): `want` cells, as many warps as they need up to what `sms` SMs hold.
+    cudaError_t launch(uint32_t lane_prec, int g, const DevArgs &A, uint32_t want, int sms, cudaStream_t s) const {
+        constexpr size_t kSmemMax = 227 * 1024;
+        const uint32_t G = kGroupLanes[g], n = head[g][0].n;
+        const GroupFn fn = lane_prec == 0 ? group_kernel_for<0>(n, G, rodas3)
+                                          : lane_prec == 1 ? group_kernel_for<1>(n, G, rodas3) : group_kernel_for<4>(n, G, rodas3);
+        const GroupArgs a = args(lane_prec, g);
+        const uint32_t need = (want + 32 / G - 1) / (32 / G);   // warps
+        // few cells: one warp per CTA, so that they spread over the SMs; else one warp per scheduler and CTA
+        uint32_t warps = need <= (uint32_t)sms ? 1u : need <= 2u * (uint32_t)sms ? 2u : 4u;
+        while (warps > 1 && smem(a, g, warps) > kSmemMax) warps >>= 1;
+        const size_t bytes = smem(a, g, warps);
+        cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        int per_sm = 0;
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, (int)(32 * warps), bytes);
+        if (e != cudaSuccess) return e;
+        if (per_sm < 1) per_sm = 1;
+        const uint32_t resident = (uint32_t)per_sm * (uint32_t)sms, ctas = (need + warps - 1) / warps;
+        fn<<<resident < ctas ? resident : ctas, 32 * warps, bytes, s>>>(A, a);
+        return cudaGetLastError();
+    }
+};
+
+}   // namespace sgb

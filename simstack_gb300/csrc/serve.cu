@@ -42,6 +42,7 @@
 #include "mech.h"
 #include "mech_tables.h"
 #include "coop.h"
+#include "group.h"
 
 namespace sgb {
 cudaError_t launch_air_p0(const Shape &, const DevArgs &, cudaStream_t);
@@ -180,6 +181,7 @@ struct Engine {
     KinMech table_mech;
     KinMethod table_method;
     bool have_table_mech = false;
+    GroupSet group[2];              // schedule images of mechanisms 0 (shipped) and 1 (table)
     void *d_coop_image = nullptr;   // mechanism 2
     CoopMech coop_head;
     KinMethod coop_method;
@@ -321,15 +323,23 @@ cudaError_t admit(Request *r) {
         return e;
     }
 
+    // precision 2 runs the module's current mixed variant (gpu_kin_set_mixed_variant), fixed at admission
+    const uint32_t mv = gpu_kin_get_mixed_variant();
+    const uint32_t kp = q.precision == 2 && mv == 1 ? 3u : q.precision == 2 && mv == 2 ? 4u : q.precision;
+    // the request's kernel: a group kernel when this and the other requests at hand leave the GPU short of
+    // cells (group_rule), else the CTA-synchronous queue, which does more cells per instruction (six
+    // requests of 2,500 cells, mixed: 53 ms, 91 ms as group kernels chosen one request at a time)
+    const GroupSet &gs = E.group[q.mechanism];
+    uint64_t at_hand = q.cells;
+    for (const Request *o : E.running) at_hand += o->desc.cells;
+    for (const Request *o : E.waiting) at_hand += o->desc.cells;
+    const int group = gs.dev ? group_rule(kp, r->generated, (uint32_t)(at_hand < 1u << 30 ? at_hand : 1u << 30), E.sms) : -1;
     Shape sh;
     sh.kind = 2;   // CTA-synchronous persistent queue
     sh.block = 128;
     sh.variant = 0;
     sh.smem = r->generated ? 0 : kTableBytes;
     int per_sm = 0;
-    // precision 2 runs the module's current mixed variant (gpu_kin_set_mixed_variant), fixed at admission
-    const uint32_t mv = gpu_kin_get_mixed_variant();
-    const uint32_t kp = q.precision == 2 && mv == 1 ? 3u : q.precision == 2 && mv == 2 ? 4u : q.precision;
     e = occupancy_chem(r->generated, kp, sh.block, sh.smem, &per_sm);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) per_sm = 1;
@@ -340,7 +350,10 @@ cudaError_t admit(Request *r) {
     // its attributes (it returns right after staging its tables)
     DevArgs idle = A;
     idle.lanes = 0;
-    e = launch_chem(r->generated, kp, sh, idle, r->stream);
+    auto chem = [&](const DevArgs &a) {
+        return group >= 0 ? gs.launch(kp, group, a, q.cells, E.sms, r->stream) : launch_chem(r->generated, kp, sh, a, r->stream);
+    };
+    e = chem(idle);
     if (e == cudaSuccess) e = cudaStreamSynchronize(r->stream);
     if (e != cudaSuccess) return e;
 
@@ -348,7 +361,7 @@ cudaError_t admit(Request *r) {
     e = cudaStreamBeginCapture(r->stream, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return e;
     cudaError_t ce = cudaMemsetAsync(r->d_scratch, 0, sizeof(uint32_t), r->stream);   // the cursor; the error flag stays sticky
-    if (ce == cudaSuccess) ce = launch_chem(r->generated, kp, sh, A, r->stream);
+    if (ce == cudaSuccess) ce = chem(A);
     if (ce == cudaSuccess)
         ce = (cudaError_t)gpu_advect(A.y, P, r->n, q.cells, q.channel_cells, r->d_inlet, r->courant, r->substeps, r->stream);
     e = cudaStreamEndCapture(r->stream, &graph);
@@ -417,6 +430,11 @@ SGB_API int32_t gpu_serve_open(uint64_t hbm_budget_bytes, const KinControl *cont
     E.graph_launches = 0;
     E.have_table_mech = false;
     E.have_coop = false;
+    KinMech air;
+    Model shipped;
+    define_air(&shipped);
+    if (shipped.finalize() && shipped.to_kinmech(&air)) e = E.group[0].build(air, true);
+    if (e != cudaSuccess) return (int32_t)e;
     E.control = control ? *control : KinControl{1e-4, 6.02214076e8, 1e-14, 0.0, 1e-9, 1000000u, 0, 1};
     E.open = true;
     return 0;
@@ -428,6 +446,8 @@ SGB_API int32_t gpu_serve_set_mech(const KinMech *mech, const KinMethod *method)
     if (!E.running.empty() || !E.waiting.empty()) return (int32_t)cudaErrorNotReady;   // requests hold the old tables
     E.table_mech = *mech;
     E.table_method = *method;
+    const cudaError_t e = E.group[1].build(*mech, method_is_rodas3(method));
+    if (e != cudaSuccess) return (int32_t)e;
     E.have_table_mech = true;
     return 0;
 }
@@ -646,5 +666,6 @@ SGB_API int32_t gpu_serve_close(void) {
     if (E.d_coop_image) cudaFree(E.d_coop_image);
     E.d_coop_image = nullptr;
     E.have_coop = false;
+    for (GroupSet &s : E.group) s.release();
     return (int32_t)cudaDeviceSynchronize();
 }
