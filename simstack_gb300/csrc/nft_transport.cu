@@ -6,14 +6,22 @@
 //
 // Data: device copies of the reference's group arrays in the reference's byte layout
 // (nft.cpp:134-203: groups of 8 channels, every per-cell quantity a [8] f32 lane array),
-// packed group after group. One CTA per group; thread (lane l, chunk q) owns a contiguous
-// run of cells of channel l. Within a substep the reference sweeps outlet -> inlet so
+// packed group after group. Within a substep the reference sweeps outlet -> inlet so
 // that every cell reads its upstream neighbour's value from before the substep; the cells
-// of a substep are therefore independent, and each thread sweeps its own run the same way
-// (outlet end first). The one value a run needs from outside is the old state of the
-// previous run's last cell: it is published in shared memory (double-buffered by
-// substep parity) before the sweep, so a substep costs one CTA barrier. A warp covers 4
-// runs x 8 lanes: each field access is four full 32-byte sectors.
+// of a substep are therefore independent, and each thread sweeps its own run of cells the
+// same way (outlet end first). The one value a run needs from outside is the old state of
+// the previous run's last cell.
+//
+// Two kernels. nft_resident_kernel (channels of up to 2,304 cells) holds a channel in the
+// registers of a warp, or of several: each lane keeps a run of kRun cells (nine fields and
+// four coefficients each) for the whole window and takes its upstream value by shuffle, so
+// a substep touches no memory but the plant sites' shared-memory slots and needs no barrier
+// while one warp holds the channel. It is bound by its own instruction issue (~30 per cell
+// and ~56 per site and substep). nft_transport_kernel keeps the state in global memory (L1)
+// and one CTA per group, the boundary values in shared memory with one barrier per substep:
+// longer channels, and runs whose site slots do not fit. 512 channels x 240 cells x 253
+// substeps: 990 us through memory (3.9 us per substep: load latency and the barrier), 184 us
+// resident (0.73 us).
 //
 // Every element receives the reference's f32 operations in the reference's order, issued
 // as explicit PTX (no contraction, no reassociation). The reference runs the transport
@@ -202,12 +210,235 @@ __global__ void __launch_bounds__(1024) nft_transport_kernel(const __grid_consta
     }
 }
 
-// Runs per channel and cells per run: as many runs as a 1,024-thread CTA holds, then
-// runs of equal length (the last may be shorter).
+// A channel in registers: kWpc = blockDim / 32 / (channels per CTA) warps hold one channel, lane i of
+// warp p the slots (32 p + i) kRun .. + kRun; the channel's cells fill the LAST slots, so its outlet is
+// always the last lane's last slot and the unused slots stay zero, as the inflow delta is (the
+// reference's inlet update is the general one with an upstream of 0, bit for bit). Slots of one
+// warp's neighbour come through shared memory (double-buffered by substep parity, one barrier).
+// site_slots: sites at most in a lane's run; shared memory: [site_slots][16][threads] drop and
+// removed, then [2][warps][9] boundary values and the evaporation carry.
+constexpr int kMaxRun = 9;
+constexpr uint32_t kMaxResidentWarps = 8;      // 255 registers a thread
+
+template <bool kFtz, int kRun>
+__global__ void __launch_bounds__(256) nft_resident_kernel(const __grid_constant__ GpuNftTransport t, uint32_t wpc,
+                                                           uint32_t site_slots) {
+    using F = F32<kFtz>;
+    extern __shared__ float sm[];
+    const uint32_t threads = blockDim.x, warps = threads / 32, warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const uint32_t part = warp % wpc, channel = blockIdx.x * (warps / wpc) + warp / wpc;
+    const bool live = channel < t.groups * kLanes;   // whole warps
+    const uint32_t g = live ? channel / kLanes : 0u, l = channel % kLanes;
+    const uint32_t cells = t.cells, pad = wpc * 32 * kRun - cells;
+    const uint32_t slot0 = (part * 32 + lane) * kRun;
+    float *rows = t.rows + (size_t)g * cells * kRow + l;
+    float *hot = t.hot + (size_t)g * cells * kHot + l;
+    const float *cold = t.cold + (size_t)g * cells * kCold + l;
+    float *sites = t.sites + (size_t)g * t.sites_count * kSite + l;
+    float *site_sm = sm + threadIdx.x;
+    float *edge = sm + (size_t)site_slots * 16 * threads;   // [2][warps][9]
+    float *carry = edge + 2 * warps * kFields;              // [warps]
+
+    float v[kRun][kFields], c[kRun], kT[kRun], bT[kRun], ko[kRun];
+    uint32_t valid = 0, on = 0;   // slots that hold a cell; cells with a plant site
+    const float tamb_rel = F::sub(t.T_amb, t.ref[kFieldT]);
+#pragma unroll
+    for (int j = 0; j < kRun; ++j) {
+        c[j] = kT[j] = bT[j] = ko[j] = 0.0f;
+#pragma unroll
+        for (uint32_t k = 0; k < kFields; ++k) v[j][k] = 0.0f;
+        if (!live || slot0 + j < pad) continue;
+        const uint32_t cell = slot0 + j - pad;
+        valid |= 1u << j;
+        // this window's heat coefficients, linear in the cell temperature delta (nft.cpp:1036-1047)
+        const float *cd = cold + (size_t)cell * kCold;
+        float *h = hot + (size_t)cell * kHot;
+        const float kw = cd[kColdKW], ge = cd[kColdGE], kr = cd[kColdKR];
+        kT[j] = F::fma(ge, t.es_slope, kw);
+        bT[j] = F::fnma(ge, t.e0, F::fma(kw, tamb_rel, F::mul(kr, t.radiant)));
+        h[kHotKT] = kT[j];
+        h[kHotBT] = bT[j];
+        c[j] = h[kHotC];
+        ko[j] = h[kHotKO];
+#pragma unroll
+        for (uint32_t k = 0; k < kFields; ++k) v[j][k] = rows[(size_t)cell * kRow + k * kLanes];
+        const int site = site_on(cell, t);
+        if (site >= 0) {
+            const uint32_t at = __popc(on);
+            on |= 1u << j;
+            const float *sr = sites + (size_t)site * kSite;
+#pragma unroll
+            for (uint32_t k = 1; k < kFields; ++k) {
+                site_sm[(at * 16 + k - 1) * threads] = sr[kSiteDrop + k * kLanes];
+                site_sm[(at * 16 + 7 + k) * threads] = sr[kSiteRemoved + k * kLanes];
+            }
+        }
+    }
+    const uint32_t any = __reduce_or_sync(0xffffffffu, on);   // slots where some lane has a site
+    const float refT = t.ref[kFieldT], refDO = t.ref[kFieldDO];
+    float out[kFields];
+#pragma unroll
+    for (uint32_t k = 0; k < kFields; ++k) out[k] = 0.0f;
+
+    for (uint32_t s = 0; s < t.substeps; ++s) {
+        float in[kFields];   // the old state upstream of slot 0
+#pragma unroll
+        for (uint32_t k = 0; k < kFields; ++k) {
+            out[k] = F::add(out[k], v[kRun - 1][k]);   // kept by the outlet's lane
+            in[k] = __shfl_up_sync(0xffffffffu, v[kRun - 1][k], 1);
+        }
+        if (wpc > 1) {
+            float *e = edge + (s & 1) * warps * kFields;
+            if (lane == 31)
+#pragma unroll
+                for (uint32_t k = 0; k < kFields; ++k) e[warp * kFields + k] = v[kRun - 1][k];
+            __syncthreads();
+            if (lane == 0)
+#pragma unroll
+                for (uint32_t k = 0; k < kFields; ++k) in[k] = part ? e[(warp - 1) * kFields + k] : 0.0f;
+        } else if (lane == 0) {
+#pragma unroll
+            for (uint32_t k = 0; k < kFields; ++k) in[k] = 0.0f;
+        }
+#pragma unroll
+        for (int j = kRun - 1; j >= 0; --j) {
+            float x[kFields];
+#pragma unroll
+            for (uint32_t k = 0; k < kFields; ++k) {
+                const float up = j ? v[j ? j - 1 : 0][k] : in[k];
+                x[k] = F::fma(c[j], F::sub(up, v[j][k]), v[j][k]);
+            }
+            // heat: walls, radiant load, evaporative cooling of the open surface
+            x[kFieldT] = F::add(F::fnma(kT[j], x[kFieldT], x[kFieldT]), bT[j]);
+            // O2 exchange with the gully air (saturation at the absolute temperature)
+            x[kFieldDO] = F::fma(ko[j], F::sub(do_sat<kFtz>(F::add(refT, x[kFieldT])), F::add(refDO, x[kFieldDO])), x[kFieldDO]);
+            // plant site: uptake and root respiration, booked as what was actually removed
+            if ((any >> j) & 1u) {   // the same for the whole warp
+                if ((on >> j) & 1u) {
+                    float *sr = site_sm + __popc(on & ((1u << j) - 1u)) * 16 * threads;
+                    float drop[kFields], removed[kFields];   // all loads ahead of the stores
+#pragma unroll
+                    for (uint32_t k = 1; k < kFields; ++k) {
+                        drop[k] = sr[(k - 1) * threads];
+                        removed[k] = sr[(7 + k) * threads];
+                    }
+#pragma unroll
+                    for (uint32_t k = 1; k < kFields; ++k) {
+                        const float before = x[k];
+                        x[k] = F::max(F::sub(x[k], drop[k]), -t.ref[k]);
+                        sr[(7 + k) * threads] = F::add(removed[k], F::sub(before, x[k]));
+                    }
+                }
+            }
+            const bool cell = (valid >> j) & 1u;   // a slot without a cell keeps its zeros whatever the air is
+            x[kFieldT] = cell ? x[kFieldT] : 0.0f;
+            x[kFieldDO] = cell ? x[kFieldDO] : 0.0f;
+#pragma unroll
+            for (uint32_t k = 0; k < kFields; ++k) v[j][k] = x[k];
+        }
+    }
+    float ev[kRun], e[kRun];
+#pragma unroll
+    for (int j = 0; j < kRun; ++j) {
+        ev[j] = e[j] = 0.0f;
+        if (!((valid >> j) & 1u)) continue;
+        const uint32_t cell = slot0 + j - pad;
+#pragma unroll
+        for (uint32_t k = 0; k < kFields; ++k) rows[(size_t)cell * kRow + k * kLanes] = v[j][k];
+        ev[j] = cold[(size_t)cell * kCold + kColdEV];
+        e[j] = F::fma(t.es_slope, v[j][kFieldT], t.e0);
+        if ((on >> j) & 1u) {
+            float *sr = sites + (size_t)site_on(cell, t) * kSite;
+            const float *from = site_sm + __popc(on & ((1u << j) - 1u)) * 16 * threads;
+#pragma unroll
+            for (uint32_t k = 1; k < kFields; ++k) sr[kSiteRemoved + k * kLanes] = from[(7 + k) * threads];
+        }
+    }
+    const bool outlet = live && part + 1 == wpc && lane == 31;
+    if (outlet)
+#pragma unroll
+        for (uint32_t k = 0; k < kFields; ++k) t.out_sum[(size_t)g * kRow + k * kLanes + l] = out[k];
+    // water evaporated from the film this window, summed inlet -> outlet (nft.cpp:1101-1105): lane by
+    // lane, warp by warp
+    float evap = 0.0f;
+    for (uint32_t p = 0; p < wpc; ++p) {
+        if (part == p) {
+            if (p) evap = carry[warp - 1];
+            for (int i = 0; i < 32; ++i) {
+                if ((int)lane == i)
+#pragma unroll
+                    for (int j = 0; j < kRun; ++j)
+                        if ((valid >> j) & 1u) evap = F::fma(ev[j], e[j], evap);
+                evap = __shfl_sync(0xffffffffu, evap, i);
+            }
+            if (lane == 0) carry[warp] = evap;
+        }
+        if (wpc > 1) __syncthreads();
+    }
+    if (outlet) t.evap_kg[(size_t)g * kLanes + l] = F::mul(evap, (float)t.substeps);
+}
+
+// Runs per channel and cells per run of nft_transport_kernel: as many runs as a 1,024-thread CTA
+// holds, then runs of equal length (the last may be shorter).
 void launch_shape(uint32_t cells, uint32_t *runs, uint32_t *run_len) {
     const uint32_t len = (cells + kMaxRuns - 1) / kMaxRuns;
     *run_len = len;
     *runs = (cells + len - 1) / len;
+}
+
+// Shape of nft_resident_kernel: cells per lane, warps per channel, channels per CTA, site slots per lane.
+struct Resident {
+    uint32_t run, wpc, channels, slots;
+    size_t smem;
+};
+// The run with the least estimated time per substep: instructions of a warp (30 per slot, 64 per slot
+// that has a site in some lane -- one per stride where the stride divides the run, so that every
+// lane has its sites at the same slots, else every slot -- and the exchange) times 2.5 + 1.75 x
+// (warps per scheduler) cycles, times the waves. Fitted to 240 cells, sites every 3, 253 substeps, us at runs of
+// 2 / 3 / 6 / 9: one group 103 / 101 / 181 / 228, 64 groups 242 / 184 / 237 / 241; it also picks
+// the best of 2..9 measured for 24 to 1,500 cells with strides 1, 3 and 7 to within 15 %.
+// False: the channel or its site slots do not fit.
+bool resident_shape(const GpuNftTransport &t, uint32_t sms, Resident *best) {
+    constexpr uint32_t kRegs[kMaxRun + 1] = {0, 0, 64, 107, 94, 109, 128, 229, 255, 255};
+    const uint32_t stride = t.sites_count > 1 ? t.site_stride : 0u;
+    double least = 0.0;
+    best->run = 0;
+    for (uint32_t run = 2; run <= (uint32_t)kMaxRun; ++run) {
+        Resident r;
+        r.run = run;
+        r.wpc = (t.cells + 32 * run - 1) / (32 * run);
+        if (r.wpc > kMaxResidentWarps) continue;
+        r.channels = r.wpc >= 4 ? 1u : 4u / r.wpc;
+        const uint32_t warps = r.wpc * r.channels;
+        r.slots = t.sites_count == 0 ? 0u : stride == 0 ? 1u : (run + stride - 1) / stride;
+        r.smem = ((size_t)r.slots * 16 * 32 * warps + 2 * warps * kFields + warps) * sizeof(float);
+        if (r.smem > 200 * 1024) continue;
+        const uint32_t blocks = t.sites_count == 0 ? 0u : stride == 0 ? 1u : run % stride == 0 ? run / stride : run;
+        const double instr = 30.0 * run + 64.0 * blocks + (r.wpc > 1 ? 40.0 : 10.0);
+        const uint32_t by_regs = 65536u / (kRegs[run] * 32u * warps), by_smem = (uint32_t)(227 * 1024 / (r.smem + 1024));
+        const uint32_t fit = by_regs < by_smem ? (by_regs ? by_regs : 1u) : (by_smem ? by_smem : 1u);
+        const uint32_t ctas = (t.groups * kLanes + r.channels - 1) / r.channels, per_sm = (ctas + sms - 1) / sms;
+        const uint32_t busy = per_sm < fit ? per_sm : fit, waves = (per_sm + fit - 1) / fit;
+        const double time = waves * instr * (2.5 + 1.75 * ((busy * warps + 3) / 4));
+        if (best->run == 0 || time < least) {
+            *best = r;
+            least = time;
+        }
+    }
+    return best->run != 0;
+}
+
+template <bool kFtz> void (*resident_kernel(uint32_t run))(GpuNftTransport, uint32_t, uint32_t) {
+    switch (run) {
+        case 2: return nft_resident_kernel<kFtz, 2>;
+        case 3: return nft_resident_kernel<kFtz, 3>;
+        case 4: return nft_resident_kernel<kFtz, 4>;
+        case 5: return nft_resident_kernel<kFtz, 5>;
+        case 6: return nft_resident_kernel<kFtz, 6>;
+        case 7: return nft_resident_kernel<kFtz, 7>;
+        case 8: return nft_resident_kernel<kFtz, 8>;
+        default: return nft_resident_kernel<kFtz, kMaxRun>;
+    }
 }
 
 bool aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0; }
@@ -223,6 +454,22 @@ SGB_API int32_t gpu_nft_transport(const GpuNftTransport *t, float *kernel_ms) {
         return (int32_t)cudaErrorInvalidValue;
     if (!aligned16(t->rows) || !aligned16(t->hot) || !aligned16(t->cold) || (t->sites && !aligned16(t->sites)))
         return (int32_t)cudaErrorInvalidValue;
+    int dev = 0, sms = 0;
+    cudaError_t q = cudaGetDevice(&dev);
+    if (q == cudaSuccess) q = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (q != cudaSuccess) return (int32_t)q;
+    Resident r;
+    if (t->groups <= 0x0fffffffu && resident_shape(*t, (uint32_t)sms, &r)) {   // the channel count fits the grid
+        auto kernel = t->flush_denormals ? resident_kernel<true>(r.run) : resident_kernel<false>(r.run);
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r.smem);
+        if (e == cudaSuccess) e = module_mark_start();
+        if (e != cudaSuccess) return (int32_t)e;
+        kernel<<<(t->groups * kLanes + r.channels - 1) / r.channels, 32 * r.wpc * r.channels, r.smem, module_stream()>>>(*t, r.wpc,
+                                                                                                                        r.slots);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return (int32_t)e;
+        return (int32_t)module_finish(kernel_ms);
+    }
     uint32_t runs = 0, run_len = 0;
     launch_shape(t->cells, &runs, &run_len);
     const uint32_t threads = runs * kLanes;
