@@ -239,8 +239,8 @@ SGB_API int32_t gpu_kin_set_mixed_variant(uint32_t variant);
 /* Straggler hand-off for precision 0 (0 = off; default 600): in one advance, a cell still
  * stepping after `attempts` step attempts on its lane is parked and finished right after by a
  * group kernel (a warp per cell), so a few very stiff cells no longer run alone on single lanes
- * at the end of the launch; the results keep the same bits. The mixed lane kernels keep their
- * cells. */
+ * at the end of the launch; the results keep the same bits. While it is on, a CTA of the queue
+ * kernel (FP64, and the default mixed variant) also parks its last few cells once the queue is dry. */
 SGB_API int32_t gpu_kin_set_straggler_budget(uint32_t attempts);
 /* Per-thread stack (local memory) reservation of the current context: set it when set_bytes
  * is nonzero; *current receives the value in force. */

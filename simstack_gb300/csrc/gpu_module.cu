@@ -177,19 +177,42 @@ struct AdvanceShape {
     GpuKinTuning t;
 };
 
+// The lane kernels' shape for the shipped mechanism, from one GB300 (ms):
+//   f32: one cell per lane to completion, 64 threads per CTA: the queue kernels' votes and barriers cost
+//     more than the refilling gives (pulsed zones, static / CTA queue: 64 zones 20.6 / 32.3, 4,096 zones
+//     20.8 / 33.0, 65,536 zones 21.0 / 22.0)
+//   mixed: once one 128-lane CTA per SM is full, one CTA of 256, whose eight warps fetch the step code
+//     together (128 x 2 / 256 threads: 16,384 cells 26.7 / 32.2, 32,768 41.5 / 33.0, 262,144 228 / 143)
+void lane_rule(uint32_t lp, uint32_t lanes, GpuKinTuning *t) {
+    if (lp == 1) *t = GpuKinTuning{0u, 64u, 0u, 0u, 0.0f};
+    if (lp == 4 && lanes > 128u * (uint32_t)g.sms) *t = GpuKinTuning{2u, 256u, 0u, 2u, 0.0f};
+}
+
 // The shape of an advance of `lanes` cells: the caller's tuning where one was set or measured,
 // else by size. A lane kernel takes as long for one cell per SM as for a full warp of them (shipped
 // mechanism, 1 s: FP64 59 ms, mixed 25 ms up to 16,384 cells), so small batches go to the group
 // kernels (group_rule in group.h).
 AdvanceShape shape_for(uint32_t prec, uint32_t lanes, bool with_mode) {
     AdvanceShape s = {-1, with_mode ? tuning_for(prec) : g.tuning[prec]};
-    if (g.tuned[prec] || (with_mode && g.mode == 1) || s.t.kind == 3 || !g.group.dev) return s;
-    s.group = group_rule(lane_prec(prec), g.generated, lanes, g.sms);
+    if (g.tuned[prec] || (with_mode && g.mode == 1) || s.t.kind == 3) return s;
+    if (g.group.dev) s.group = group_rule(lane_prec(prec), g.generated, g.mech.species_count, lanes, g.sms);
+    if (s.group < 0 && g.generated) lane_rule(lane_prec(prec), lanes, &s.t);
     return s;
 }
 
-// Whether a lane advance of this precision hands its stragglers on.
-bool handoff(uint32_t prec) { return g.straggler_budget && g.group.dev && prec == 0; }
+// Whether a lane advance of this precision hands cells on: stragglers (FP64) and the last ones of the
+// CTA queue kernel (FP64 and the default mixed variant).
+bool handoff(uint32_t prec) { return g.straggler_budget && g.group.dev && (lane_prec(prec) == 0 || lane_prec(prec) == 4); }
+
+// Cells at which a CTA of the queue kernel parks what it has left: where its attempt costs what a
+// group kernel takes for as many cells at full throughput. Shipped mechanism, cycles: FP64 lanes
+// 308k per 128-lane attempt against ~9.3k per cell and attempt of 8-lane groups (33 cells), mixed
+// 149k per 256 lanes against ~6.5k (23); the table lanes take ~2M per 128, so any CTA that is not full parks.
+uint32_t drain_at(uint32_t prec, const GpuKinTuning &t) {
+    if (t.kind != 2) return 0;
+    if (!g.generated) return t.block - 1;
+    return lane_prec(prec) == 0 ? t.block / 4 : t.block / 11;
+}
 
 // The group kernel on cells of `A` (its cursor is zeroed first), or on the parked ones (A.resume).
 cudaError_t launch_group(uint32_t prec, int group, const DevArgs &A0, cudaStream_t stream) {
@@ -239,7 +262,8 @@ cudaError_t launch_advance(uint32_t prec, const AdvanceShape &s, const DevArgs &
     }
     if (!handoff(prec)) return launch_lanes(prec, t, A0);
     DevArgs A = A0;
-    A.budget = g.straggler_budget;
+    A.budget = prec == 0 ? g.straggler_budget : 0;
+    A.drain = drain_at(prec, t);
     A.suspend_cap = kSuspendCap;
     A.suspend_count = g.d_suspend_count;
     A.suspend = g.d_suspend;
@@ -623,7 +647,7 @@ SGB_API int32_t gpu_kin_advance_pipelined(const GpuKinLaunch *launch, void *host
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&g.kern2, cudaStreamNonBlocking);
         if (e != cudaSuccess) return (int32_t)e;
     }
-    const bool serial = handoff(launch->precision);
+    const bool serial = handoff(launch->precision) && launch->precision == 0;
     const uint64_t P = launch->padded, lanes = launch->lane_count ? launch->lane_count : launch->padded;
     const uint64_t pitch = P * sizeof(double);
     const uint64_t per = (lanes + chunks - 1) / chunks;
@@ -648,7 +672,7 @@ SGB_API int32_t gpu_kin_advance_pipelined(const GpuKinLaunch *launch, void *host
         Lc.lane_count = (uint32_t)count;
         DevArgs A;
         fill_args(&Lc, &A);
-        const AdvanceShape shape = shape_for(launch->precision, A.lanes, false);
+        const AdvanceShape shape = shape_for(launch->precision, serial ? A.lanes : (uint32_t)lanes, false);
         if (serial) {
             e = launch_advance(launch->precision, shape, A);
         } else {

@@ -34,16 +34,20 @@ constexpr uint32_t kGroupLanes[3] = {8, 16, 32};
 //                    2,048 cells: FP64 20.9 / 16.7 / 20.1 / 59.4   mixed 12.2 / 11.0 / 14.4 / 25.3
 //                    4,096 cells: FP64 34.2 / 25.8 / 23.2 / 59.5   mixed 18.6 / 16.5 / 16.2 / 25.4
 //                    8,192 cells: FP64 62.7 / 44.3 / 35.4 / 59.4   mixed 33.0 / 26.5 / 23.9 / 24.8
-//                   16,384 cells: FP64  -  /  -  / 57.9 / 59.7     mixed  -  /  -  / 37.3 / 24.4
-//   24 species / 80 reactions, 1,501 cells: FP64 21.4 / 26.3 / 25.3 / 378   mixed 16.7 / 13.1 / 22.3 / 485
-// (the table-driven lane kernels keep a cell's arrays in local memory: ~1 ms per attempt).
-inline int group_rule(uint32_t lane_prec, bool generated, uint32_t lanes, int sms) {
+//                   10,240 cells: FP64 8 lanes 41.7, lane kernel with its hand-off 46.6; 14,336: 52.2, 45.6
+//                    6,144 cells: mixed 8 lanes 21.2, lane kernel with its hand-off 21.9; 7,168: 22.8, 21.7
+// The table-driven lane kernels keep a cell's arrays in local memory (~1 ms per attempt) and win only
+// where they fill the GPU several times over (0.1 s, 65,536 cells, 8 lanes / lane kernel): FP64 8 species
+// 54 / 51, 16 species 176 / 203, 24 species 513 / 576, 32 species 16,384 cells 339 / 372 and 65,536
+// cells 1,287 / 929 (its cells leave room for three warps per SM); mixed 38 / 50, 118 / 239, 445 / 688.
+inline int group_rule(uint32_t lane_prec, bool generated, uint32_t n, uint32_t lanes, int sms) {
     const uint32_t c = (lanes + (uint32_t)sms - 1) / (uint32_t)sms;
     if (lane_prec != 0 && lane_prec != 1 && lane_prec != 4) return -1;   // the other mixed variants: lanes only
+    if (generated && lane_prec == 1) return -1;   // f32 lanes are as fast from one zone on (64 zones pulsed: 20.6 against 22.2)
     if (c <= (lane_prec == 4 ? 10u : 8u)) return 2;
-    if (generated && lane_prec == 1) return c <= 12u ? 1 : -1;
     if (c <= (lane_prec == 4 ? 26u : 16u)) return 1;
-    return c <= (!generated ? 128u : lane_prec == 4 ? 48u : 96u) ? 0 : -1;
+    if (generated) return c <= (lane_prec == 4 ? 42u : 78u) ? 0 : -1;
+    return lane_prec != 0 || c <= (n > 24 ? 128u : 400u) ? 0 : -1;
 }
 
 // One mechanism's schedule images on the device: per lanes-per-cell and lane precision (0 FP64, 1 f32
@@ -115,7 +119,7 @@ struct GroupSet {
         const uint32_t need = (want + 32 / G - 1) / (32 / G);   // warps
         // few cells: one warp per CTA, so that they spread over the SMs; else one warp per scheduler and CTA
         uint32_t warps = need <= (uint32_t)sms ? 1u : need <= 2u * (uint32_t)sms ? 2u : 4u;
-        while (warps > 1 && smem(a, g, warps) > kSmemMax) warps >>= 1;
+        while (warps > 1 && smem(a, g, warps) > kSmemMax) --warps;
         const size_t bytes = smem(a, g, warps);
         cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
         int per_sm = 0;

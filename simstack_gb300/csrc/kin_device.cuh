@@ -143,6 +143,7 @@ struct DevArgs {
     // `budget` step attempts in this launch parks its scalar state in `suspend` and leaves; a
     // group kernel finishes it (0 = never). Group kernels: a warp with such a cell stops claiming.
     uint32_t budget;
+    uint32_t drain;            // CTA queue kernel: a CTA down to this many cells parks them (the queue is dry then)
     uint32_t suspend_cap;
     uint32_t *suspend_count;
     struct SuspendRec *suspend;
@@ -287,6 +288,7 @@ struct Lane {
         phase = kPhaseSegStart;
     }
 
+    static constexpr bool kParks = PREC == 0;
     // Straggler hand-off: park the scalar state; false if the list is full (the lane keeps the cell).
     __device__ __forceinline__ bool park(const DevArgs &A, uint32_t cell) {
         const uint32_t slot = atomicAdd(A.suspend_count, 1u);
@@ -304,6 +306,8 @@ struct Lane {
         phase = kPhaseDone;
         return true;
     }
+
+    __device__ __forceinline__ void store_parked(const DevArgs &A, uint32_t i) { store(A, i); }
 
     // dbd_lanes.h:60-77: f32 lanes add their increment to the f64 storage.
     __device__ __forceinline__ void store(const DevArgs &A, uint32_t i) {
@@ -641,6 +645,7 @@ __device__ __forceinline__ Df df_prod_f(float a, float b) {   // exact product o
 // consecutive banks), instead of in the lane's registers / local memory.
 template <class Ops, class M, int kLuStride = 0>
 struct LaneDf {
+    static constexpr bool kParks = false;
     static constexpr int N = Ops::N, R = Ops::R, NNZ = Ops::NNZ, S = M::kStages;
     static constexpr size_t kSmemBytes = kLuStride ? (size_t)NNZ * kLuStride * sizeof(float) : 0;
 
@@ -1024,6 +1029,7 @@ struct LaneIr {
     static constexpr bool kPhaseBarriers = SGB_IR_PHASE_BARRIERS != 0, kStageBarriers = SGB_IR_STAGE_BARRIERS != 0;
     static constexpr int N = Ops::N, R = Ops::R, NNZ = Ops::NNZ, S = M::kStages;
     static constexpr size_t kSmemBytes = kLuStride ? (size_t)NNZ * kLuStride * sizeof(float) : 0;
+    static constexpr bool kParks = true;
     static constexpr bool kTmemK = kTmemCols > 0;
     static constexpr uint32_t kTmemAlloc = (uint32_t)kTmemCols;
     static_assert(!kTmemK || (2 * N <= 64 && S * 64 <= 256), "stage vectors must fit 64 TMEM columns each, 4 stages");
@@ -1136,11 +1142,32 @@ struct LaneIr {
             if (s >= (int)nn) break;
             A.y[(size_t)s * p + i] = df_to(Df{yhi[s], ylo[s]});
         }
+        store_records(A, i);
+    }
+    __device__ __forceinline__ void store_records(const DevArgs &A, uint32_t i) {
         A.h[i] = h;
         A.failed[i] = failed;
         A.steps[i] += steps;
         A.rejects[i] += rejects;
         A.pulses[i] += pulses;
+    }
+    // As Lane::park; the state goes to the y slots as its float pairs (a double cannot hold every
+    // pair), which the group kernel that resumes the cell reads back and stores as doubles.
+    __device__ __forceinline__ bool park(const DevArgs &A, uint32_t cell) {
+        const uint32_t slot = atomicAdd(A.suspend_count, 1u);
+        if (slot >= A.suspend_cap) return false;
+        A.suspend[slot] = SuspendRec{t, h, seg_end, applied, cell, iterations, transitions,
+                                     (pending ? 1u : 0u) | (reject_last ? 2u : 0u) | (reject_more ? 4u : 0u)};
+        phase = kPhaseDone;
+        return true;
+    }
+    __device__ __forceinline__ void store_parked(const DevArgs &A, uint32_t i) {
+        const uint32_t p = A.padded, nn = n();
+        for (int s = 0; s < N; ++s) {
+            if (s >= (int)nn) break;
+            ((Df *)A.y)[(size_t)s * p + i] = Df{yhi[s], ylo[s]};
+        }
+        store_records(A, i);
     }
 
     __device__ __forceinline__ void seg_start(const DevArgs &A) {

@@ -170,7 +170,9 @@ __global__ void __launch_bounds__(Budget<V>::kThreads, Budget<V>::kMinBlocks) ki
 // the straight-line step code instead of one stretch each (the step code is
 // far larger than the instruction caches). Lanes without a cell compute on
 // their last state and commit nothing; a lane that never had one starts from
-// a copy of cell 0.
+// a copy of cell 0. An attempt costs the CTA the same however few of its lanes
+// have a cell, so once the queue is dry a CTA down to A.drain cells parks
+// them for a group kernel (kin_group.cuh) and leaves.
 template <class Ops, class M, int PREC, int V>
 __global__ void __launch_bounds__(Budget<V>::kThreads, Budget<V>::kMinBlocks) kin_queue_cta_kernel(const __grid_constant__ DevArgs A) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -205,7 +207,24 @@ __global__ void __launch_bounds__(Budget<V>::kThreads, Budget<V>::kMinBlocks) ki
             L.store(A, cell);
             have = false;
         }
-        if (!__syncthreads_or(need)) break;
+        if constexpr (decltype(L)::kParks) {
+            const int active = __syncthreads_count(need);
+            if (active == 0) break;
+            if ((uint32_t)active <= A.drain) {   // fewer cells than lanes: the queue is dry
+                if (need) {
+                    --L.iterations;   // the attempt that was due is counted again where the cell resumes
+                    if (L.park(A, cell)) {
+                        L.store_parked(A, cell);
+                        have = need = false;
+                    } else {
+                        ++L.iterations;
+                    }
+                }
+                if (!__syncthreads_or(need)) break;
+            }
+        } else if (!__syncthreads_or(need)) {
+            break;
+        }
         L.template attempt<true>(A, need);
     }
     lanes_tmem_close<decltype(L)>(&tmem_slot);

@@ -333,7 +333,7 @@ cudaError_t admit(Request *r) {
     uint64_t at_hand = q.cells;
     for (const Request *o : E.running) at_hand += o->desc.cells;
     for (const Request *o : E.waiting) at_hand += o->desc.cells;
-    const int group = gs.dev ? group_rule(kp, r->generated, (uint32_t)(at_hand < 1u << 30 ? at_hand : 1u << 30), E.sms) : -1;
+    const int group = gs.dev ? group_rule(kp, r->generated, r->n, (uint32_t)(at_hand < 1u << 30 ? at_hand : 1u << 30), E.sms) : -1;
     Shape sh;
     sh.kind = 2;   // CTA-synchronous persistent queue
     sh.block = 128;

@@ -107,3 +107,24 @@ def test_failed_and_subset_lanes(untuned, oracle_lib):
     assert_bits(z, ref)
     assert z["failed"].sum() > 0
     untuned.reset_arena()
+
+
+@pytest.mark.parametrize("precision,cells", [(0, 12001), (2, 6501), (2, 19999), (1, 5001)])
+def test_large_batches_by_rule(untuned, cells, precision):
+    """Past the group kernels' range: the lane shapes the rule picks, whose last cells are parked and resumed
+    (FP64, mixed), against the warp-synchronous queue, which parks none with the hand-off off."""
+    ctl = DBD_CTL if precision == 1 else {}
+    z = sg.air_cells(cells, seed=7)
+    ref = z.copy()
+    untuned.set_mech(sg.Model.air().kinmech(), sg.method("rodas3"), sg.control(**ctl))
+    dur = 1e-4 if precision == 1 else 0.3
+    untuned.integrate(z, dur, precision=precision)
+    if precision != 1:
+        assert untuned.parked_cells() > 0
+    untuned.reset_arena()
+    untuned.set_straggler_budget(0)
+    untuned.set_tuning(kind=1)
+    untuned.integrate(ref, dur, precision=precision)
+    untuned.set_straggler_budget(sg.DEFAULT_STRAGGLER_BUDGET)
+    sg.check(sg.lib().gpu_init(0, 2 << 30, untuned.info), "gpu_init")   # untuned again
+    assert_bits(z, ref)
