@@ -75,14 +75,9 @@ __device__ unsigned long long g_coop_phase_cycles[8];
 #define SGB_PHASE(i, stmt) stmt
 #endif
 
-// Pivots per elimination pass of the FP64 factorisation with its LU in global memory (1, 2 or 4;
-// the same bits for any). Measured on 200 species / 1,200 reactions, 1,216 cells x 2 s, 256
-// threads x 2 CTAs per SM: 1 -> 6,817 ms, 2 -> 5,805 ms, 4 -> 6,272 ms (the one-warp panel grows).
-// The shared-memory LUs (FP64 of small mechanisms, the mixed path's FP32) stay pivot by pivot:
-// the mixed kernel measured 2,392 ms pivot by pivot against 2,745 (2) and 2,630 (4).
-#ifndef SGB_COOP_PIVOT_BLOCK
-#define SGB_COOP_PIVOT_BLOCK 2
-#endif
+// Species from which the elimination runs in panels (a thread per row: CTAs of at least n threads);
+// below, and in smaller CTAs, pivot by pivot.
+constexpr uint32_t kCoopPanelMin = 40;
 
 // Shared-memory doubles before the mixed path's FP32 arrays.
 __host__ __device__ inline uint32_t coop_smem_doubles(uint32_t n, uint32_t R) { return 11u * n + 2u * R + 8u; }
@@ -266,12 +261,10 @@ struct CoopCell {
     // l(i,k) = a[i][k] * (1/U(k,k)) and stores it once the row is done, so a pivot
     // needs one barrier (FP32) or two (FP64: the shared inverse).
     __device__ void factor(Cf ghinv) {
-#if SGB_COOP_PIVOT_BLOCK > 1
-        if (!kMixed && lu_global) {
-            factor_block<SGB_COOP_PIVOT_BLOCK>(ghinv);
+        if (n >= kCoopPanelMin && NT >= n) {
+            factor_panels<kMixed ? 8 : 4>(ghinv);
             return;
         }
-#endif
         for (uint32_t k = 0; k < n; ++k) {
             const uint32_t nl = lcnt[k];
             Cf inv;
@@ -353,107 +346,141 @@ struct CoopCell {
         sync();
     }
 
-    // B pivots per pass (k .. k+B-1). Panel: warp 0 gives each row r of the block the updates of
-    // the block's pivots before it, in order, then takes 1/U(r,r), and stages row r's U part in
-    // shared memory. Trailing rows i >= k+B, one warp per row: the row's block entries become its
-    // multipliers in order (a[i][k+p] takes the updates of pivots k+q, q < p, then the scaling by
-    // 1/U(k+p,k+p)), and each a[i][j], j >= k+B, takes the block's pivots' updates in ascending
-    // order, loaded once and stored once. Every element receives the operations of the pivot-by-
-    // pivot order, in that order, with 1/B of the passes over the trailing rows (the LU of a large
-    // mechanism lives in L2) and of the barriers. The staged rows use the stage vectors K (free
-    // until the stages begin) and the inverses red[4..7], so B <= 4.
+    // B pivots per pass (k .. k+B-1), one thread per row in the panel:
+    //   panel     thread i holds row i's B block entries; pivot by pivot the pivot row's thread takes
+    //             1/U and publishes its entries, and every row below forms its multiplier and takes the
+    //             update of the block's later columns
+    //   U rows    one thread per column right of the block: the block's rows take each other's
+    //             updates (loaded ahead of the panel)
+    //   trailing  a warp per row, 32 columns at a time with the block's U entries in registers: every
+    //             element is loaded and stored once and takes the block's updates in ascending order
+    // Every element receives the operations of the pivot-by-pivot order, in that order. What this buys
+    // over a pivot (FP32) or two (FP64) per pass: a row's multiplier is one instruction per 32 rows and not
+    // one per row (FP64: a third of the instructions of the unit that bounds it), and the trailing
+    // elements make 1/B of the trips to shared memory (FP32) or L2 (FP64). The buffers are the
+    // stage vectors K (multipliers) and the four vectors after them (U rows), free until the
+    // stages begin, so B is 4 in FP64 and 8 in FP32; the pattern words use x32. Measured on 200 species /
+    // 1,200 reactions, cycles per factorisation: FP64 one CTA per SM 3.05M -> 1.90M, two (per pair of
+    // cells) 2.77M of 2.5M that its FP64 instructions take at the unit's rate; FP32 550k -> 357k.
     template <uint32_t B>
-    __device__ void factor_block(Cf ghinv) {
-        static_assert(B >= 1 && B <= 4 && 32 % B == 0, "block of 1, 2 or 4 pivots");
-        static_assert(kCoopMaxCols * B <= 32, "column masks in one word");
+    __device__ void factor_panels(Cf ghinv) {
+        static_assert(B * sizeof(Cf) <= 32, "panel buffers: 32 bytes per row in K, and as much for the U rows");
         Cf *inv_s = (Cf *)(red + 4);
-        Cf *u = (Cf *)K;   // [B][n] staged pivot rows, zero off the pattern
+        Cf *Lp = (Cf *)K;        // [row][B]
+        Cf *Up = (Cf *)ytmp;     // [B][column]
+        uint16_t *live = (uint16_t *)x32, *rows_on = live + kCoopMaxSpecies;   // pattern bits per column / row of the block
         for (uint32_t k = 0; k < n; k += B) {
-            const uint32_t nb = n - k < B ? n - k : B;
-            if (warp == 0) {   // the panel
-                for (uint32_t r = k; r < k + nb; ++r) {
-                    Cf *rr = a + (size_t)r * ld;
-                    for (uint32_t q = k; q < r; ++q) {
-                        if (!bit(r, q)) continue;   // same for the whole warp
-                        const Cf l = rr[q] * inv_s[q - k];
-                        const Cf *uq = u + (size_t)(q - k) * n;
-                        for (uint32_t j = q + 1 + lane; j < n; j += 32)
-                            if (bit(q, j)) rr[j] = sgb_fma(-l, uq[j], rr[j]);
-                        __syncwarp();
-                        if (lane == 0) rr[q] = l;
-                        __syncwarp();
-                    }
-                    if (lane == 0) {
-                        const Cf v = (Cf)1.0 / (rr[r] + ghinv);
-                        rr[r] = v;
-                        inv_s[r - k] = v;
-                    }
-                    __syncwarp();
-                    Cf *ur = u + (size_t)(r - k) * n;
-                    for (uint32_t j = r + 1 + lane; j < n; j += 32) ur[j] = bit(r, j) ? rr[j] : (Cf)0.0;
-                    __syncwarp();
-                }
+            const uint32_t nb = n - k < B ? n - k : B, j0 = k + nb;
+            const uint32_t mine = (1u << nb) - 1u;
+            // row tid of the panel
+            const bool row_in = tid >= k && tid < n;
+            uint32_t bm = 0;
+            Cf pa[B];
+            if (row_in) {
+                bm = (pat[tid * 8u + (k >> 5)] >> (k & 31u)) & mine;   // k is a multiple of B: one word
+#pragma unroll
+                for (uint32_t p = 0; p < B; ++p) pa[p] = p < nb ? a[(size_t)tid * ld + k + p] : (Cf)0.0;
             }
-            sync();
-            const uint32_t j0 = k + nb;
-            if (j0 >= n) break;
-            const uint32_t bmask = (1u << nb) - 1u;
-            // per lane: which block pivots update column j0 + lane + 32c (bits c*B + p)
-            uint32_t live = 0;
-#pragma unroll
-            for (uint32_t c = 0; c < kCoopMaxCols; ++c) {
-                const uint32_t j = j0 + lane + 32u * c;
-                if (j >= n) continue;
-#pragma unroll
-                for (uint32_t p = 0; p < B; ++p)
-                    if (p < nb && bit(k + p, j)) live |= 1u << (c * B + p);
-            }
-            // inner[p]: block pivots q < p whose row has column k+p
-            uint32_t inner = 0;
-#pragma unroll
-            for (uint32_t p = 1; p < B; ++p)
-#pragma unroll
-                for (uint32_t q = 0; q < p; ++q)
-                    if (p < nb && bit(k + q, k + p)) inner |= 1u << (p * B + q);
-            for (uint32_t i = j0 + warp; i < n; i += W) {
-                // row i's pattern bits at the block's columns (k is a multiple of B: one word)
-                const uint32_t bm = (pat[i * 8u + (k >> 5)] >> (k & 31u)) & bmask;
-                if (!bm) continue;   // same for the whole warp
-                Cf *row = a + (size_t)i * ld;
-                Cf l[B];
+            // column j0 + tid of the U rows, loaded ahead
+            const uint32_t j = j0 + tid;
+            uint32_t lv = 0;
+            Cf ux[B];
+            if (j < n) {
 #pragma unroll
                 for (uint32_t p = 0; p < B; ++p) {
-                    l[p] = (Cf)0.0;
-                    if ((bm >> p) & 1u) {
-                        Cf x = row[k + p];
-#pragma unroll
-                        for (uint32_t q = 0; q < p; ++q)
-                            if (((bm >> q) & 1u) && ((inner >> (p * B + q)) & 1u)) x = sgb_fma(-l[q], u[(size_t)q * n + k + p], x);
-                        l[p] = x * inv_s[p];
+                    ux[p] = (Cf)0.0;
+                    if (p < nb && bit(k + p, j)) {
+                        lv |= 1u << p;
+                        ux[p] = a[(size_t)(k + p) * ld + j];
                     }
                 }
-                Cf v[kCoopMaxCols];
+            }
 #pragma unroll
-                for (uint32_t c = 0; c < kCoopMaxCols; ++c) {
-                    const uint32_t j = j0 + lane + 32u * c;
-                    v[c] = (Cf)0.0;
-                    if ((live >> (c * B)) & bm) v[c] = row[j];
+            for (uint32_t p = 0; p < B; ++p) {
+                if (p >= nb) break;
+                const uint32_t kp = k + p;
+                if (tid == kp) {
+                    const Cf v = (Cf)1.0 / (pa[p] + ghinv);
+#pragma unroll
+                    for (uint32_t q = 0; q < B; ++q) Lp[kp * B + q] = pa[q];
+                    inv_s[p & 3u] = v;
+                    pa[p] = v;
                 }
+                sync();
+                if (tid > kp && row_in && ((bm >> p) & 1u)) {
+                    const Cf l = pa[p] * inv_s[p & 3u];
+                    pa[p] = l;
+                    const uint32_t on = (pat[kp * 8u + (k >> 5)] >> (k & 31u)) & mine;   // row kp's columns in the block
 #pragma unroll
-                for (uint32_t c = 0; c < kCoopMaxCols; ++c) {
-                    const uint32_t j = j0 + lane + 32u * c;
-                    const uint32_t m = (live >> (c * B)) & bm;
-                    if (!m) continue;
-                    Cf x = v[c];
-#pragma unroll
-                    for (uint32_t p = 0; p < B; ++p)
-                        if ((m >> p) & 1u) x = sgb_fma(-l[p], u[(size_t)p * n + j], x);
-                    row[j] = x;
+                    for (uint32_t q = p + 1; q < B; ++q)
+                        if ((on >> q) & 1u) pa[q] = sgb_fma(-l, Lp[kp * B + q], pa[q]);
                 }
-                __syncwarp();   // every lane has read the block entries
+            }
+            if (row_in) {
 #pragma unroll
                 for (uint32_t p = 0; p < B; ++p)
-                    if (lane == p && ((bm >> p) & 1u)) row[k + p] = l[p];
+                    if (p < nb) a[(size_t)tid * ld + k + p] = pa[p];
+                if (tid >= j0) {
+#pragma unroll
+                    for (uint32_t p = 0; p < B; ++p) Lp[tid * B + p] = pa[p];
+                    rows_on[tid] = (uint16_t)bm;
+                }
+            }
+            if (j0 >= n) break;
+            if (j < n) {
+#pragma unroll
+                for (uint32_t p = 1; p < B; ++p) {
+                    const uint32_t lo = (pat[(k + p) * 8u + (k >> 5)] >> (k & 31u)) & lv;
+#pragma unroll
+                    for (uint32_t q = 0; q < p; ++q)
+                        if ((lo >> q) & 1u) ux[p] = sgb_fma(-Lp[(k + p) * B + q], ux[q], ux[p]);
+                }
+#pragma unroll
+                for (uint32_t p = 0; p < B; ++p) {
+                    if ((lv >> p) & 1u) a[(size_t)(k + p) * ld + j] = ux[p];
+                    Up[p * n + j] = ux[p];
+                }
+                live[j] = (uint16_t)lv;
+            }
+            sync();
+            for (uint32_t c = j0; c < n; c += 32) {
+                const uint32_t jc = c + lane;
+                const bool on = jc < n;
+                const uint32_t lc = on ? live[jc] : 0u;
+                const uint32_t any = __reduce_or_sync(0xffffffffu, lc);
+                if (!any) continue;
+                const bool full = __all_sync(0xffffffffu, !on || lc == mine);
+                Cf u[B];
+#pragma unroll
+                for (uint32_t p = 0; p < B; ++p) u[p] = on ? Up[p * n + jc] : (Cf)0.0;
+                for (uint32_t i = j0 + warp; i < n; i += 4 * W) {   // four rows at a time: their loads overlap
+                    uint32_t b[4];
+                    Cf v[4];
+#pragma unroll
+                    for (uint32_t r = 0; r < 4; ++r) {   // b: the same for the whole warp
+                        const uint32_t ii = i + r * W;
+                        b[r] = ii < n ? rows_on[ii] & any : 0u;
+                        v[r] = (Cf)0.0;
+                        if (b[r] && on) v[r] = a[(size_t)ii * ld + jc];
+                    }
+#pragma unroll
+                    for (uint32_t r = 0; r < 4; ++r) {
+                        if (!b[r]) continue;
+                        const uint32_t ii = i + r * W;
+                        const Cf *lp = Lp + ii * B;
+                        if (full && b[r] == mine) {
+#pragma unroll
+                            for (uint32_t p = 0; p < B; ++p) v[r] = sgb_fma(-lp[p], u[p], v[r]);
+                            if (on) a[(size_t)ii * ld + jc] = v[r];
+                        } else {
+                            const uint32_t m = b[r] & lc;
+#pragma unroll
+                            for (uint32_t p = 0; p < B; ++p)
+                                if ((m >> p) & 1u) v[r] = sgb_fma(-lp[p], u[p], v[r]);
+                            if (m) a[(size_t)ii * ld + jc] = v[r];
+                        }
+                    }
+                }
             }
             sync();
         }
@@ -794,15 +821,15 @@ __global__ void __launch_bounds__(512, 1) kin_coop_kernel(const __grid_constant_
     C.warp = threadIdx.x >> 5;
     C.W = blockDim.x >> 5;
     const uint32_t n = C.n;
-    C.y = sm;
-    C.ytmp = C.y + n;
-    C.fcn = C.ytmp + n;
-    C.src = C.fcn + n;
-    C.qv = C.src + n;
+    C.K = sm;   // 4 stage vectors; with the four vectors after them the elimination's panel buffers
+    C.ytmp = C.K + 4 * n;
+    C.qv = C.ytmp + n;
     C.rb = C.qv + n;
     C.xv = C.rb + n;
-    C.K = C.xv + n;   // 4 stage vectors
-    C.kr = C.K + 4 * n;
+    C.y = C.xv + n;
+    C.fcn = C.y + n;
+    C.src = C.fcn + n;
+    C.kr = C.src + n;
     C.rate = C.kr + C.R;
     C.red = C.rate + C.R;
     C.x32 = (float *)(sm + coop_smem_doubles(n, C.R));
