@@ -37,10 +37,6 @@ struct CoopMech {
     uint32_t bytes;           // image size
     // byte offsets from the image start (each 16-byte aligned)
     uint32_t off_reac;        // uint16[R][4]: reactant count, then up to 3 reactant species
-    uint32_t off_fbeg;        // uint32[n+1]
-    uint32_t off_fent;        // CoopTerm[fun_terms], per species, reactions ascending
-    uint32_t off_jbeg;        // uint32[nj+1]
-    uint32_t off_jent;        // CoopTerm[jac_terms], per entry, (r, p, e) ascending
     uint32_t off_jpos;        // uint32[nj]: row * ld + col
     uint32_t off_jrow;        // uint32[n+1]: entries of row i are [jrow[i], jrow[i+1])
     uint32_t off_jcol;        // uint16[nj]
@@ -52,7 +48,24 @@ struct CoopMech {
     uint32_t off_crow;        // uint16[]: rows i < k with (i, k) in the filled pattern, per column k
     uint32_t off_pat;         // uint32[n][8]: filled pattern, bit j of row i (n <= 256)
     uint32_t off_lcnt;        // uint16[n]: rows below the diagonal in column k
+    uint32_t pairs;           // (reaction, reactant) pairs
+    // what the kernels walk: the products k_r prod_{q != p} y_q once per pair, and the RHS and Jacobian
+    // terms in groups of 32 lists of like length (longest first), term k of a group's lists side by
+    // side: coalesced reads, and a warp waits for no list much longer than its others
+    uint32_t off_pair;        // uint2[pairs]: r | count << 24, s0 | s1 << 16 (the other reactants)
+    uint32_t off_fgrp;        // uint2[(n + 31) / 32]: first term, terms
+    uint32_t off_fdst;        // uint32[32 per group]: species (~0: none)
+    uint32_t off_fterm;       // CoopWide[]: reaction
+    uint32_t off_jgrp;        // uint2[(nj + 31) / 32]
+    uint32_t off_jdst;        // uint2[32 per group]: row * ld + col (~0: none), entry index
+    uint32_t off_jterm;       // CoopWide[]: pair
     uint32_t reserved;
+};
+
+// A term of the grouped lists: the high word of its coefficient as a double (the low one is 0: small
+// integers), so that no conversion is needed. Lists shorter than their group end in index ~0.
+struct CoopWide {
+    uint32_t index, hi;
 };
 
 }   // namespace sgb

@@ -3,6 +3,8 @@
 // reference-layout KinMech (the same pattern, slots and scatter lists).
 #include <string.h>
 
+#include <algorithm>
+
 #include "coop.h"
 #include "mech.h"
 
@@ -99,13 +101,7 @@ bool build_image(const Desc &d, std::vector<uint8_t> *out) {
     std::vector<std::vector<CoopTerm>> fs(n);
     for (uint32_t r = 0; r < R; ++r)
         for (auto &e : d.net[r]) fs[e.first].push_back({r, (float)e.second});
-    std::vector<uint32_t> fbeg(n + 1, 0);
-    std::vector<CoopTerm> fent;
-    for (uint32_t s = 0; s < n; ++s) {
-        fbeg[s] = (uint32_t)fent.size();
-        fent.insert(fent.end(), fs[s].begin(), fs[s].end());
-    }
-    fbeg[n] = (uint32_t)fent.size();
+    for (uint32_t i = 0; i < n; ++i) h.fun_terms += (uint32_t)fs[i].size();
     // Jacobian terms per compact slot, (r, p, e) ascending; entries = slots some reaction scatters into
     std::vector<std::vector<CoopTerm>> js(d.nnz);
     for (uint32_t r = 0; r < R; ++r)
@@ -124,19 +120,16 @@ bool build_image(const Desc &d, std::vector<uint8_t> *out) {
                 slot_col[s] = j;
             }
         }
-    std::vector<uint32_t> jbeg, jpos, jrow(n + 1, 0);
+    std::vector<uint32_t> jpos, jrow(n + 1, 0);
     std::vector<uint16_t> jcol;
-    std::vector<CoopTerm> jent;
     for (uint32_t s = 0; s < d.nnz; ++s) {   // slots are row-major, so entries come out sorted by row
         if (js[s].empty()) continue;
-        jbeg.push_back((uint32_t)jent.size());
-        jent.insert(jent.end(), js[s].begin(), js[s].end());
+        h.jac_terms += (uint32_t)js[s].size();
         jpos.push_back(slot_row[s] * h.ld + slot_col[s]);
         jcol.push_back((uint16_t)slot_col[s]);
         jrow[slot_row[s] + 1]++;
     }
     h.nj = (uint32_t)jpos.size();
-    jbeg.push_back((uint32_t)jent.size());
     for (uint32_t i = 0; i < n; ++i) jrow[i + 1] += jrow[i];
     // elimination lists
     std::vector<uint32_t> lbeg(n + 1), ubeg(n + 1), cbeg(n + 1);
@@ -164,8 +157,70 @@ bool build_image(const Desc &d, std::vector<uint8_t> *out) {
                 pat[(size_t)i * 8 + (j >> 5)] |= 1u << (j & 31);
                 if (i > j) lcnt[j]++;
             }
-    h.fun_terms = (uint32_t)fent.size();
-    h.jac_terms = (uint32_t)jent.size();
+    // pairs and grouped lists
+    std::vector<uint32_t> pair, fgrp, fdst, jgrp, jdst;
+    std::vector<CoopWide> fterm, jterm;
+    std::vector<uint32_t> pair_at((size_t)R * 3, 0u);
+    for (uint32_t r = 0; r < R; ++r) {
+        const std::vector<uint32_t> &re = d.reactants[r];
+        if (R > 0xffffffu) return false;
+        for (size_t p = 0; p < re.size(); ++p) {
+            uint32_t other = 0, c = 0;
+            for (size_t q = 0; q < re.size(); ++q)
+                if (q != p) other |= re[q] << (16 * c++);
+            pair_at[(size_t)r * 3 + p] = (uint32_t)pair.size() / 2;
+            pair.push_back(r | c << 24);
+            pair.push_back(other);
+        }
+    }
+    h.pairs = (uint32_t)pair.size() / 2;
+    bool wide_ok = true;
+    auto wide = [&](uint32_t index, float coef) {
+        const double v = coef;
+        uint64_t b;
+        memcpy(&b, &v, 8);
+        wide_ok = wide_ok && (uint32_t)b == 0;
+        return CoopWide{index, (uint32_t)(b >> 32)};
+    };
+    // lists[order[..]] in groups of 32, longest first; dst_words words of `dst` per list
+    auto group = [&](const std::vector<std::vector<CoopWide>> &lists, const std::vector<std::vector<uint32_t>> &target,
+                     std::vector<uint32_t> *grp, std::vector<uint32_t> *dst, std::vector<CoopWide> *terms) {
+        std::vector<uint32_t> order(lists.size());
+        for (uint32_t e = 0; e < order.size(); ++e) order[e] = e;
+        std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return lists[x].size() > lists[y].size(); });
+        const size_t words = target.empty() ? 1 : target[0].size();
+        for (size_t g0 = 0; g0 < order.size(); g0 += 32) {
+            const size_t len = lists[order[g0]].size();
+            grp->push_back((uint32_t)terms->size());
+            grp->push_back((uint32_t)len);
+            for (size_t l = 0; l < 32; ++l)
+                for (size_t q = 0; q < words; ++q) dst->push_back(g0 + l < order.size() ? target[order[g0 + l]][q] : ~0u);
+            for (size_t k = 0; k < len; ++k)
+                for (size_t l = 0; l < 32; ++l) {
+                    const bool on = g0 + l < order.size() && k < lists[order[g0 + l]].size();
+                    terms->push_back(on ? lists[order[g0 + l]][k] : CoopWide{~0u, 0u});
+                }
+        }
+    };
+    {
+        std::vector<std::vector<CoopWide>> fl(n), jl;
+        std::vector<std::vector<uint32_t>> ft(n), jt;
+        for (uint32_t i = 0; i < n; ++i) {
+            ft[i] = {i};
+            for (const CoopTerm &t : fs[i]) fl[i].push_back(wide(t.index, t.coef));
+        }
+        uint32_t e = 0;
+        for (uint32_t sl = 0; sl < d.nnz; ++sl) {
+            if (js[sl].empty()) continue;
+            jt.push_back({jpos[e], e});
+            jl.push_back({});
+            for (const CoopTerm &t : js[sl]) jl.back().push_back(wide(pair_at[(size_t)(t.index & 0xffffffu) * 3 + (t.index >> 24)], t.coef));
+            ++e;
+        }
+        group(fl, ft, &fgrp, &fdst, &fterm);
+        group(jl, jt, &jgrp, &jdst, &jterm);
+        if (!wide_ok) return false;   // a net change that is no small integer
+    }
     h.l_entries = (uint32_t)lrow.size();
     h.u_entries = (uint32_t)ucol.size();
 
@@ -176,10 +231,13 @@ bool build_image(const Desc &d, std::vector<uint8_t> *out) {
         off = align16(off + bytes);
     };
     place(&h.off_reac, reac.size() * 2);
-    place(&h.off_fbeg, fbeg.size() * 4);
-    place(&h.off_fent, fent.size() * sizeof(CoopTerm));
-    place(&h.off_jbeg, jbeg.size() * 4);
-    place(&h.off_jent, jent.size() * sizeof(CoopTerm));
+    place(&h.off_pair, pair.size() * 4);
+    place(&h.off_fgrp, fgrp.size() * 4);
+    place(&h.off_fdst, fdst.size() * 4);
+    place(&h.off_fterm, fterm.size() * sizeof(CoopWide));
+    place(&h.off_jgrp, jgrp.size() * 4);
+    place(&h.off_jdst, jdst.size() * 4);
+    place(&h.off_jterm, jterm.size() * sizeof(CoopWide));
     place(&h.off_jpos, jpos.size() * 4);
     place(&h.off_jrow, jrow.size() * 4);
     place(&h.off_jcol, jcol.size() * 2);
@@ -200,10 +258,6 @@ bool build_image(const Desc &d, std::vector<uint8_t> *out) {
         if (bytes) memcpy(b + o, src, bytes);
     };
     put(h.off_reac, reac.data(), reac.size() * 2);
-    put(h.off_fbeg, fbeg.data(), fbeg.size() * 4);
-    put(h.off_fent, fent.data(), fent.size() * sizeof(CoopTerm));
-    put(h.off_jbeg, jbeg.data(), jbeg.size() * 4);
-    put(h.off_jent, jent.data(), jent.size() * sizeof(CoopTerm));
     put(h.off_jpos, jpos.data(), jpos.size() * 4);
     put(h.off_jrow, jrow.data(), jrow.size() * 4);
     put(h.off_jcol, jcol.data(), jcol.size() * 2);
@@ -215,6 +269,13 @@ bool build_image(const Desc &d, std::vector<uint8_t> *out) {
     put(h.off_crow, crow.data(), crow.size() * 2);
     put(h.off_pat, pat.data(), pat.size() * 4);
     put(h.off_lcnt, lcnt.data(), lcnt.size() * 2);
+    put(h.off_pair, pair.data(), pair.size() * 4);
+    put(h.off_fgrp, fgrp.data(), fgrp.size() * 4);
+    put(h.off_fdst, fdst.data(), fdst.size() * 4);
+    put(h.off_fterm, fterm.data(), fterm.size() * sizeof(CoopWide));
+    put(h.off_jgrp, jgrp.data(), jgrp.size() * 4);
+    put(h.off_jdst, jdst.data(), jdst.size() * 4);
+    put(h.off_jterm, jterm.data(), jterm.size() * sizeof(CoopWide));
     return true;
 }
 

@@ -36,27 +36,23 @@ constexpr uint32_t kCoopMaxCols = kCoopMaxSpecies / 32;
 struct CoopTab {
     const CoopMech *h;
     const uint16_t *reac;
-    const uint32_t *fbeg, *jbeg, *jpos, *jrow, *lbeg, *ubeg, *cbeg;
-    const CoopTerm *fent, *jent;
-    const uint16_t *jcol, *lrow, *ucol, *crow;
+    const uint2 *pair, *fgrp, *fterm, *jgrp, *jdst, *jterm;
+    const uint32_t *fdst, *jrow;
+    const uint16_t *jcol;
 
-    __device__ __forceinline__ void init(const void *image) {
-        const unsigned char *b = (const unsigned char *)image;
-        h = (const CoopMech *)b;
-        reac = (const uint16_t *)(b + h->off_reac);
-        fbeg = (const uint32_t *)(b + h->off_fbeg);
-        fent = (const CoopTerm *)(b + h->off_fent);
-        jbeg = (const uint32_t *)(b + h->off_jbeg);
-        jent = (const CoopTerm *)(b + h->off_jent);
-        jpos = (const uint32_t *)(b + h->off_jpos);
-        jrow = (const uint32_t *)(b + h->off_jrow);
-        jcol = (const uint16_t *)(b + h->off_jcol);
-        lbeg = (const uint32_t *)(b + h->off_lbeg);
-        lrow = (const uint16_t *)(b + h->off_lrow);
-        ubeg = (const uint32_t *)(b + h->off_ubeg);
-        ucol = (const uint16_t *)(b + h->off_ucol);
-        cbeg = (const uint32_t *)(b + h->off_cbeg);
-        crow = (const uint16_t *)(b + h->off_crow);
+    // at: where the image's byte 0 lies, or would (the lists may be staged elsewhere than the header)
+    __device__ __forceinline__ void init(const CoopMech *head, const unsigned char *at) {
+        h = head;
+        reac = (const uint16_t *)(at + h->off_reac);
+        pair = (const uint2 *)(at + h->off_pair);
+        fgrp = (const uint2 *)(at + h->off_fgrp);
+        fdst = (const uint32_t *)(at + h->off_fdst);
+        fterm = (const uint2 *)(at + h->off_fterm);
+        jgrp = (const uint2 *)(at + h->off_jgrp);
+        jdst = (const uint2 *)(at + h->off_jdst);
+        jterm = (const uint2 *)(at + h->off_jterm);
+        jrow = (const uint32_t *)(at + h->off_jrow);
+        jcol = (const uint16_t *)(at + h->off_jcol);
     }
 };
 
@@ -105,6 +101,13 @@ __host__ __device__ inline CoopSmemLayout coop_layout(int prec, const CoopMech &
     return L;
 }
 
+// Whether the Jacobian's products fit the shared-memory vectors that are free while it is formed, and the
+// CTA's scratch before them: the FP64 LU, or the mixed path's Jacobian entries.
+__host__ __device__ inline bool coop_products_fit(const CoopMech &h) { return h.pairs <= 8u * h.n + h.R; }
+__host__ __device__ inline size_t coop_scratch_base(int prec, const CoopMech &h) {
+    return prec == 2 ? (size_t)h.nj : (size_t)h.n * h.ld;
+}
+
 template <int PREC>
 struct CoopCell {
     typedef typename Pick<PREC == 0, double, float>::type Cf;   // LU and solve arithmetic
@@ -120,6 +123,7 @@ struct CoopCell {
     const uint32_t *pat;    // shared: filled pattern, 8 words per row
     const uint16_t *lcnt;   // shared: rows below the diagonal per column
     double *js;     // mixed: Jacobian entries (a = -J) in FP64
+    double *prod;   // the Jacobian's products
     // replicated scalar state (kin_solver.h:189-345)
     double t, h, seg_end, applied, duration, period, first, count, steps, rejects, pulses, failed;
     uint32_t iterations, transitions;
@@ -212,44 +216,93 @@ struct CoopCell {
         }
     }
 
+    // acc = fma(coef, from[index], acc) over this lane's list of a group (coop.h), four terms at a time so
+    // that their loads overlap.
+    __device__ __forceinline__ double gather(double acc, const uint2 *term, uint32_t len, const double *from) const {
+        for (uint32_t k = 0; k < len; k += 4) {
+            uint2 t[4];
+            double v[4];
+#pragma unroll
+            for (uint32_t q = 0; q < 4; ++q) t[q] = k + q < len ? term[(k + q) * 32u] : make_uint2(~0u, 0u);
+#pragma unroll
+            for (uint32_t q = 0; q < 4; ++q) v[q] = t[q].x != ~0u ? from[t[q].x] : 0.0;
+#pragma unroll
+            for (uint32_t q = 0; q < 4; ++q)
+                if (t[q].x != ~0u) acc = sgb_fma(__hiloint2double((int)t[q].y, 0), v[q], acc);
+        }
+        return acc;
+    }
+
     // fcn = f(yy): rates per reaction, then each species' terms in reaction order.
     __device__ void rhs(const double *yy) {
-        for (uint32_t r = tid; r < R; r += NT) {
-            const uint16_t *rc = tb.reac + (size_t)r * 4;
-            double v = kr[r];
-            for (uint32_t p = 0; p < rc[0]; ++p) v = v * yy[rc[1 + p]];
-            rate[r] = v;
+        const uint2 *words = (const uint2 *)tb.reac;   // count, s0 | s1 << 16 in 16-bit fields
+        for (uint32_t r0 = tid; r0 < R; r0 += 4 * NT) {
+            uint2 w[4];
+            double v[4];
+#pragma unroll
+            for (uint32_t q = 0; q < 4; ++q) {
+                const uint32_t r = r0 + q * NT;
+                w[q] = r < R ? words[r] : make_uint2(0u, 0u);
+                v[q] = r < R ? kr[r] : 0.0;
+            }
+#pragma unroll
+            for (uint32_t q = 0; q < 4; ++q) {
+                const uint32_t c = w[q].x & 0xffffu;
+                if (c > 0) v[q] = v[q] * yy[w[q].x >> 16];
+                if (c > 1) v[q] = v[q] * yy[w[q].y & 0xffffu];
+                if (c > 2) v[q] = v[q] * yy[w[q].y >> 16];
+                if (r0 + q * NT < R) rate[r0 + q * NT] = v[q];
+            }
         }
         sync();
-        for (uint32_t s = tid; s < n; s += NT) {
-            double f = src[s];
-            for (uint32_t e = tb.fbeg[s]; e < tb.fbeg[s + 1]; ++e) {
-                const CoopTerm term = tb.fent[e];
-                f = sgb_fma((double)term.coef, rate[term.index], f);
-            }
-            fcn[s] = f;
+        for (uint32_t g = warp; g < (n + 31) / 32; g += W) {
+            const uint2 range = tb.fgrp[g];
+            const uint32_t s = tb.fdst[g * 32 + lane];
+            const double f = gather(s != ~0u ? src[s] : 0.0, tb.fterm + range.x + lane, range.y, rate);
+            if (s != ~0u) fcn[s] = f;
         }
         sync();
     }
 
-    // a = -J at yy (zero elsewhere); mixed: the FP64 entries also kept in js.
+    // a = -J at yy (zero elsewhere); mixed: the FP64 entries also kept in js. The products
+    // k_r prod_{q != p} y_q are formed once per (reaction, reactant) in `prod` (the panel buffers and the
+    // rates' array, or the CTA's scratch where they do not fit) and summed per entry in (r, p, e)
+    // order, entries of like length to a warp (200 species: 230k -> 40k cycles FP64, 130k -> 20k mixed,
+    // where every term formed its own product behind four dependent table reads).
     __device__ void neg_jac(const double *yy) {
-        const uint32_t total = n * ld;
-        for (uint32_t q = tid; q < total; q += NT) a[q] = (Cf)0.0;
-        sync();
-        for (uint32_t e = tid; e < nj; e += NT) {
-            double acc = 0.0;
-            for (uint32_t q = tb.jbeg[e]; q < tb.jbeg[e + 1]; ++q) {
-                const CoopTerm term = tb.jent[q];
-                const uint32_t r = term.index & 0xffffffu, p = term.index >> 24;
-                const uint16_t *rc = tb.reac + (size_t)r * 4;
-                double d = kr[r];
-                for (uint32_t o = 0; o < rc[0]; ++o)
-                    if (o != p) d = d * yy[rc[1 + o]];
-                acc = sgb_fma((double)term.coef, d, acc);
+        if (kMixed || !lu_global) {
+            uint2 *z = (uint2 *)a;   // 8-byte aligned
+            const uint32_t words = n * ld * (uint32_t)sizeof(Cf) / 8u;
+            for (uint32_t q = tid; q < words; q += NT) z[q] = make_uint2(0u, 0u);
+            if (tid == 0 && sizeof(Cf) == 4 && ((n * ld) & 1u)) a[n * ld - 1] = (Cf)0.0;
+        } else {
+            double2 *z = (double2 *)a;
+            for (uint32_t q = tid; q < n * ld / 2; q += NT) z[q] = make_double2(0.0, 0.0);
+            if (tid == 0 && ((n * ld) & 1u)) a[n * ld - 1] = (Cf)0.0;
+        }
+        const uint32_t pairs = tb.h->pairs;
+        for (uint32_t q0 = tid; q0 < pairs; q0 += 4 * NT) {
+            uint2 w[4];
+            double v[4];
+#pragma unroll
+            for (uint32_t q = 0; q < 4; ++q) w[q] = q0 + q * NT < pairs ? tb.pair[q0 + q * NT] : make_uint2(0u, 0u);
+#pragma unroll
+            for (uint32_t q = 0; q < 4; ++q) v[q] = R ? kr[w[q].x & 0xffffffu] : 0.0;
+#pragma unroll
+            for (uint32_t q = 0; q < 4; ++q) {
+                const uint32_t c = w[q].x >> 24;
+                if (c > 0) v[q] = v[q] * yy[w[q].y & 0xffffu];
+                if (c > 1) v[q] = v[q] * yy[w[q].y >> 16];
+                if (q0 + q * NT < pairs) prod[q0 + q * NT] = v[q];
             }
-            if constexpr (kMixed) js[e] = acc;
-            a[tb.jpos[e]] = (Cf)acc;
+        }
+        sync();
+        for (uint32_t g = warp; g < (nj + 31) / 32; g += W) {
+            const uint2 range = tb.jgrp[g], to = tb.jdst[g * 32 + lane];
+            const double acc = gather(0.0, tb.jterm + range.x + lane, range.y, prod);
+            if (to.x == ~0u) continue;
+            if constexpr (kMixed) js[to.y] = acc;
+            a[to.x] = (Cf)acc;
         }
         sync();
     }
@@ -262,7 +315,8 @@ struct CoopCell {
     // needs one barrier (FP32) or two (FP64: the shared inverse).
     __device__ void factor(Cf ghinv) {
         if (n >= kCoopPanelMin && NT >= n) {
-            factor_panels<kMixed ? 8 : 4>(ghinv);
+            if constexpr (kMixed) factor_panels_f32(ghinv);
+            else factor_panels<4>(ghinv);
             return;
         }
         for (uint32_t k = 0; k < n; ++k) {
@@ -487,29 +541,286 @@ struct CoopCell {
         sync();
     }
 
-    // Row elements [k0, min(k0 + kSolveBatch, end)) of a block's pattern columns, loaded together
-    // ahead of the FMA chain that uses them (the LU of a large mechanism lives in L2).
-    static constexpr uint32_t kSolveBatch = 8;
-    __device__ __forceinline__ static void load_batch(Cf (&r)[kSolveBatch], const Cf *row, uint32_t k0, uint32_t end,
-                                                      uint32_t w) {
+    // factor_panels in FP32, B = 8, without pattern tests: an element off the pattern is zero and stays
+    // zero, and a product with it changes no value. The block's rows lie in one warp, which
+    // factors them by shuffle (a reciprocal, one shuffle per entry), so a panel needs two barriers and
+    // not one per pivot; trailing rows are walked 64 columns at a time, the multipliers of a row
+    // (two 16-byte broadcasts) serving sixteen FMAs per lane. 357k cycles per factorisation of 200
+    // species with the FP64 panels' pattern tests and barriers, 175k so.
+    static __device__ __forceinline__ void load8(float (&out)[8], const float *from) {   // 16-byte aligned
+        const float4 lo = ((const float4 *)from)[0], hi = ((const float4 *)from)[1];
+        out[0] = lo.x; out[1] = lo.y; out[2] = lo.z; out[3] = lo.w;
+        out[4] = hi.x; out[5] = hi.y; out[6] = hi.z; out[7] = hi.w;
+    }
+    __device__ void factor_panels_f32(float ghinv) {
+        constexpr uint32_t B = 8;
+        float *A32 = (float *)a, *Lp = (float *)K, *Up = (float *)ytmp;
+        for (uint32_t k = 0; k < n; k += B) {
+            const uint32_t nb = n - k < B ? n - k : B, j0 = k + nb, j = j0 + tid, w0 = k >> 5, base = k & 31u;
+            const bool row_in = tid >= k && tid < n;
+            float pa[B], ux[B];
 #pragma unroll
-        for (uint32_t q = 0; q < kSolveBatch; ++q) {
-            r[q] = (Cf)0.0;
-            if (k0 + q < end && ((w >> (k0 + q)) & 1u)) r[q] = row[k0 + q];
+            for (uint32_t p = 0; p < B; ++p) {
+                pa[p] = row_in && p < nb ? A32[(size_t)tid * ld + k + p] : 0.0f;
+                ux[p] = j < n && p < nb ? A32[(size_t)(k + p) * ld + j] : 0.0f;
+            }
+            if (warp == w0) {
+#pragma unroll
+                for (uint32_t p = 0; p < B; ++p) {
+                    if (p >= nb) break;
+                    const float inv = 1.0f / (__shfl_sync(0xffffffffu, pa[p], base + p) + ghinv);
+                    const float l = pa[p] * inv;
+#pragma unroll
+                    for (uint32_t q = p + 1; q < B; ++q) {
+                        const float u = __shfl_sync(0xffffffffu, pa[q], base + p);
+                        if (lane > base + p) pa[q] = sgb_fma(-l, u, pa[q]);
+                    }
+                    pa[p] = lane > base + p ? l : lane == base + p ? inv : pa[p];
+                }
+                if (lane >= base && lane < base + nb) {
+#pragma unroll
+                    for (uint32_t p = 0; p < B; ++p) Lp[tid * B + p] = pa[p];
+                }
+            }
+            sync();
+            if (row_in && warp > w0) {
+#pragma unroll
+                for (uint32_t p = 0; p < B; ++p) {
+                    if (p >= nb) break;
+                    float up[B];
+                    load8(up, Lp + (k + p) * B);
+                    const float l = pa[p] * up[p];
+                    pa[p] = l;
+#pragma unroll
+                    for (uint32_t q = p + 1; q < B; ++q) pa[q] = sgb_fma(-l, up[q], pa[q]);
+                }
+            }
+            if (row_in) {
+#pragma unroll
+                for (uint32_t p = 0; p < B; ++p)
+                    if (p < nb) A32[(size_t)tid * ld + k + p] = pa[p];
+                if (tid >= j0) {
+#pragma unroll
+                    for (uint32_t p = 0; p < B; ++p) Lp[tid * B + p] = pa[p];
+                }
+            }
+            if (j0 >= n) break;
+            if (j < n) {
+#pragma unroll
+                for (uint32_t p = 1; p < B; ++p)
+#pragma unroll
+                    for (uint32_t q = 0; q < p; ++q) ux[p] = sgb_fma(-Lp[(k + p) * B + q], ux[q], ux[p]);
+#pragma unroll
+                for (uint32_t p = 0; p < B; ++p) {
+                    A32[(size_t)(k + p) * ld + j] = ux[p];
+                    Up[p * n + j] = ux[p];
+                }
+            }
+            sync();
+            for (uint32_t c = j0; c < n; c += 64) {
+                const uint32_t c0 = c + lane, c1 = c0 + 32;
+                const bool on0 = c0 < n, on1 = c1 < n;
+                float u0[B], u1[B];
+                bool any = false;
+#pragma unroll
+                for (uint32_t p = 0; p < B; ++p) {
+                    u0[p] = on0 ? Up[p * n + c0] : 0.0f;
+                    u1[p] = on1 ? Up[p * n + c1] : 0.0f;
+                    any = any || u0[p] != 0.0f || u1[p] != 0.0f;
+                }
+                if (!__any_sync(0xffffffffu, any)) continue;
+                for (uint32_t i = j0 + warp; i < n; i += 4 * W) {   // four rows at a time
+                    float v0[4], v1[4];
+#pragma unroll
+                    for (uint32_t r = 0; r < 4; ++r) {
+                        const uint32_t ii = i + r * W;
+                        if (ii >= n) break;   // the same for the whole warp
+                        const float *q = A32 + ii * ld + c0;
+                        v0[r] = on0 ? q[0] : 0.0f;
+                        v1[r] = on1 ? q[32] : 0.0f;
+                    }
+#pragma unroll
+                    for (uint32_t r = 0; r < 4; ++r) {
+                        const uint32_t ii = i + r * W;
+                        if (ii >= n) break;
+                        float lp[B];
+                        load8(lp, Lp + ii * B);
+#pragma unroll
+                        for (uint32_t p = 0; p < B; ++p) {
+                            v0[r] = sgb_fma(-lp[p], u0[p], v0[r]);
+                            v1[r] = sgb_fma(-lp[p], u1[p], v1[r]);
+                        }
+                        float *q = A32 + ii * ld + c0;
+                        if (on0) q[0] = v0[r];
+                        if (on1) q[32] = v1[r];
+                    }
+                }
+            }
+            sync();
+        }
+        sync();
+    }
+
+    // x = (LU)^-1 x in place. Forward (unit L) takes each row's columns ascending, backward (U,
+    // diagonal holding 1/U(k,k)) descending, then the diagonal.
+    template <class V>
+    __device__ void solve(V *x) {
+        if (NT < n) {
+            solve_plain(x);
+            return;
+        }
+        const uint32_t warps = (n + 31) / 32;   // the warps that hold rows; the others wait at the end
+        if (warp < warps) {
+            if constexpr (kMixed) solve_rows_f32(a, n, ld, x, 32 * warps);
+            else solve_rows(a, pat, n, ld, x, 32 * warps);
+        }
+        sync();
+    }
+
+    // A barrier among the CTA's first `threads` threads.
+    static __device__ __forceinline__ void sync_rows(uint32_t threads) { asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory"); }
+
+    // A thread per row, its x in a register, eight columns per barrier: the warp that holds those
+    // rows solves them, passing each one on through shared memory (35 cycles; the two shuffles take
+    // 64), while the rows past that warp take the eight before; every row has the next eight
+    // columns' coefficients on their way meanwhile. What is left is the chain itself: an FMA
+    // (FP64 64 cycles, backward a product before it) and the hand-over per column: 157k -> 86k
+    // cycles per FP64 solve of 200 species (one CTA per SM).
+    // (Calls of their own: inlined, the compiler spreads the registers of the whole step over them.)
+    static __device__ __noinline__ void solve_rows(const Cf *a, const uint32_t *pat, uint32_t n, uint32_t ld, double *x,
+                                                   uint32_t threads) {
+        constexpr uint32_t B = 8;
+        const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+        const uint32_t i = tid, blocks = (n + B - 1) / B;
+        const bool mine = i < n;
+        const Cf *row = a + (size_t)(mine ? i : 0) * ld;
+        const uint32_t *prow = pat + (mine ? i : 0) * 8u;
+        double xi = mine ? x[i] : 0.0;
+        Cf c[B], next[B];
+        auto load = [&](Cf (&r)[B], uint32_t k, bool need) {
+#pragma unroll
+            for (uint32_t q = 0; q < B; ++q) r[q] = need && k + q < n ? row[k + q] : (Cf)0.0;
+        };
+        auto bits = [&](uint32_t k) { return (prow[k >> 5] >> (k & 31u)) & 0xffu; };   // this row's pattern at columns k..k+7
+        load(c, 0, mine);
+        sync_rows(threads);   // x is read
+        for (uint32_t s = 0; s < blocks; ++s) {
+            const uint32_t k = s * B, w0 = k >> 5, base = k & 31u, on = bits(k);
+            load(next, k + B, mine && i > k + B);
+            if (warp == w0) {
+#pragma unroll
+                for (uint32_t q = 0; q < B; ++q) {
+                    if (k + q >= n) break;
+                    if (lane == base + q) x[k + q] = xi;
+                    __syncwarp();
+                    if (mine && lane > base + q && ((on >> q) & 1u)) xi = sgb_fma(-(double)c[q], x[k + q], xi);
+                }
+            }
+            sync_rows(threads);
+            if (warp > w0 && mine) {
+#pragma unroll
+                for (uint32_t q = 0; q < B; ++q)
+                    if (k + q < n && ((on >> q) & 1u)) xi = sgb_fma(-(double)c[q], x[k + q], xi);
+            }
+#pragma unroll
+            for (uint32_t q = 0; q < B; ++q) c[q] = next[q];
+        }
+        load(c, (blocks - 1) * B, mine);
+        for (uint32_t s = blocks; s-- > 0;) {
+            const uint32_t k = s * B, w0 = k >> 5, base = k & 31u, on = bits(k);
+            load(next, s ? k - B : 0u, mine && s && i < k);
+            if (warp == w0) {
+#pragma unroll
+                for (uint32_t q = B; q-- > 0;) {
+                    if (k + q >= n) continue;
+                    if (lane == base + q) x[k + q] = xi = xi * (double)c[q];   // all its updates are in
+                    __syncwarp();
+                    if (lane < base + q && ((on >> q) & 1u)) xi = sgb_fma(-(double)c[q], x[k + q], xi);
+                }
+            }
+            sync_rows(threads);
+            if (warp < w0) {
+#pragma unroll
+                for (uint32_t q = B; q-- > 0;)
+                    if (k + q < n && ((on >> q) & 1u)) xi = sgb_fma(-(double)c[q], x[k + q], xi);
+            }
+#pragma unroll
+            for (uint32_t q = 0; q < B; ++q) c[q] = next[q];
+        }
+    }
+    // FP32, a barrier per 32 columns: a warp solves its 32 rows by shuffle (~30 cycles a column; the barriers of
+    // eight-column blocks cost more than they spread) from coefficients it loaded once for both
+    // directions, the rows past it have theirs on their way meanwhile. No pattern or bounds tests:
+    // off the pattern the LU is zero, and so are the coefficients and x of rows past the end (x has
+    // room for whole blocks). 34k -> 24k cycles per solve of 200 species.
+    static __device__ __noinline__ void solve_rows_f32(const Cf *a, uint32_t n, uint32_t ld, float *x, uint32_t threads) {
+        constexpr uint32_t B = 32;
+        const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+        const uint32_t blocks = threads / 32;
+        const bool mine = tid < n;
+        const float *row = (const float *)a + (size_t)(mine ? tid : 0) * ld;
+        float xi = mine ? x[tid] : 0.0f;
+        float cd[B], co[B];   // this row's coefficients in its own block, and in the one being applied
+        auto load = [&](float (&r)[B], uint32_t k) {
+            if (k + B <= n) {
+#pragma unroll
+                for (uint32_t q = 0; q < B; ++q) r[q] = row[k + q];
+            } else {
+#pragma unroll
+                for (uint32_t q = 0; q < B; ++q) r[q] = k + q < n ? row[k + q] : 0.0f;
+            }
+        };
+        auto apply = [&](uint32_t k, bool up) {   // the columns of block k, ascending or descending
+            float xk[B];
+#pragma unroll
+            for (uint32_t q = 0; q < B; ++q) xk[q] = x[k + q];
+            if (up) {
+#pragma unroll
+                for (uint32_t q = 0; q < B; ++q) xi = sgb_fma(-co[q], xk[q], xi);
+            } else {
+#pragma unroll
+                for (uint32_t q = B; q-- > 0;) xi = sgb_fma(-co[q], xk[q], xi);
+            }
+            xi = mine ? xi : 0.0f;
+        };
+        load(cd, warp * B);
+        float inv = 0.0f;   // 1/U(i,i)
+#pragma unroll
+        for (uint32_t q = 0; q < B; ++q) inv = lane == q ? cd[q] : inv;
+        float ct[B];        // the own block's triangle, zero elsewhere: a step is a shuffle and an FMA
+#pragma unroll
+        for (uint32_t q = 0; q < B; ++q) ct[q] = lane > q ? cd[q] : 0.0f;
+        sync_rows(threads);   // x is read
+        for (uint32_t b = 0; b < blocks; ++b) {
+            if (warp == b) {
+#pragma unroll
+                for (uint32_t q = 0; q + 1 < B; ++q) xi = sgb_fma(-ct[q], __shfl_sync(0xffffffffu, xi, q), xi);
+                xi = mine ? xi : 0.0f;
+                x[tid] = xi;
+            } else if (warp > b) {
+                load(co, b * B);
+            }
+            sync_rows(threads);
+            if (warp > b) apply(b * B, true);
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < B; ++q) ct[q] = lane < q ? cd[q] : 0.0f;
+        for (uint32_t b = blocks; b-- > 0;) {
+            if (warp == b) {
+#pragma unroll
+                for (uint32_t q = B; q-- > 0;) xi = sgb_fma(-ct[q], __shfl_sync(0xffffffffu, xi * inv, q), xi);
+                xi = mine ? xi * inv : 0.0f;   // nothing changed a row after its own column
+                x[tid] = xi;
+            } else if (warp < b) {
+                load(co, b * B);
+            }
+            sync_rows(threads);
+            if (warp < b) apply(b * B, false);
         }
     }
 
-    // x = (LU)^-1 x in place, in 32-column blocks. Forward (unit L): a warp
-    // solves the diagonal block with shuffles, then every row below takes the
-    // block's updates in ascending column order. Backward (U, diagonal holding
-    // 1/U(k,k)): blocks from the last; rows above take the block's updates in
-    // descending column order; a row's diagonal scaling follows its last update.
-    template <class V>
-    __device__ void solve(V *x) {
-        if constexpr (kMixed) solve_plain(x);   // FP32 LU in shared memory: element by element
-        else solve_batched(x);                  // FP64 LU, in L2 for large mechanisms: batched loads
-    }
-
+    // In 32-column blocks, for CTAs of fewer threads than rows: a warp solves the diagonal block with
+    // shuffles, then every row outside it takes the block's updates.
     template <class V>
     __device__ void solve_plain(V *x) {
         const uint32_t nb = (n + 31) / 32;
@@ -572,100 +883,6 @@ struct CoopCell {
         }
     }
 
-    // solve_plain's operations in its order, each row's pattern elements of a block loaded
-    // kSolveBatch at a time ahead of the FMAs that use them (measured on the 200-species FP64
-    // case: 1.05x the whole step; the mixed path's shared-memory LU measured 1.03x slower).
-    template <class V>
-    __device__ void solve_batched(V *x) {
-        const uint32_t nb = (n + 31) / 32;
-        for (uint32_t b = 0; b < nb; ++b) {
-            const uint32_t kb = b * 32;
-            const uint32_t kend = kb + 32 < n ? kb + 32 : n;
-            const uint32_t kn = kend - kb;   // columns in this block (32, or fewer in the last)
-            if (warp == 0) {
-                const uint32_t i = kb + lane;
-                V xi = i < n ? x[i] : (V)0.0;
-                const Cf *row = a + (size_t)(i < n ? i : 0) * ld + kb;
-                // this row's pattern bits for the block's columns, below the diagonal only
-                const uint32_t w = i < n ? pat[i * 8u + b] & ((1u << lane) - 1u) : 0u;
-                for (uint32_t k0 = 0; k0 < kn; k0 += kSolveBatch) {
-                    Cf r[kSolveBatch];
-                    load_batch(r, row, k0, kn, w);
-#pragma unroll
-                    for (uint32_t q = 0; q < kSolveBatch; ++q) {
-                        if (k0 + q >= kn) break;
-                        const V xk = __shfl_sync(0xffffffffu, xi, k0 + q);
-                        if ((w >> (k0 + q)) & 1u) xi = sgb_fma(-(V)r[q], xk, xi);
-                    }
-                }
-                if (i < n) x[i] = xi;
-            }
-            sync();
-            for (uint32_t i = kend + tid; i < n; i += NT) {
-                const Cf *row = a + (size_t)i * ld + kb;
-                const uint32_t w = pat[i * 8u + b];
-                if (!w) continue;
-                V xi = x[i];
-                for (uint32_t k0 = 0; k0 < kn; k0 += kSolveBatch) {
-                    Cf r[kSolveBatch];
-                    load_batch(r, row, k0, kn, w);
-#pragma unroll
-                    for (uint32_t q = 0; q < kSolveBatch; ++q)
-                        if (k0 + q < kn && ((w >> (k0 + q)) & 1u)) xi = sgb_fma(-(V)r[q], x[kb + k0 + q], xi);
-                }
-                x[i] = xi;
-            }
-            sync();
-        }
-        for (uint32_t b = nb; b-- > 0;) {
-            const uint32_t kb = b * 32;
-            const uint32_t kend = kb + 32 < n ? kb + 32 : n;
-            const uint32_t kn = kend - kb;
-            if (warp == 0) {
-                const uint32_t i = kb + lane;
-                V xi = i < n ? x[i] : (V)0.0;
-                const Cf *row = a + (size_t)(i < n ? i : 0) * ld + kb;
-                // this row's pattern bits for the block's columns, above the diagonal only (columns < n)
-                const uint32_t w = i < n ? pat[i * 8u + b] & ~((2u << lane) - 1u) : 0u;
-                const V d = i < n ? (V)row[lane] : (V)0.0;   // 1/U(i,i)
-                // batches from the block's last column down, each in descending order
-                for (uint32_t top = kn; top > 0;) {
-                    const uint32_t k0 = top > kSolveBatch ? top - kSolveBatch : 0;
-                    Cf r[kSolveBatch];
-                    load_batch(r, row, k0, top, w);
-#pragma unroll
-                    for (uint32_t q = kSolveBatch; q-- > 0;) {
-                        if (k0 + q >= top) continue;
-                        const uint32_t kk = k0 + q;
-                        if (lane == kk) xi = xi * d;   // row kb+kk: all its updates are in
-                        const V xk = __shfl_sync(0xffffffffu, xi, kk);
-                        if ((w >> kk) & 1u) xi = sgb_fma(-(V)r[q], xk, xi);
-                    }
-                    top = k0;
-                }
-                if (i < n) x[i] = xi;
-            }
-            sync();
-            for (uint32_t i = tid; i < kb; i += NT) {
-                const Cf *row = a + (size_t)i * ld + kb;
-                const uint32_t w = pat[i * 8u + b];
-                if (!w) continue;
-                V xi = x[i];
-                for (uint32_t top = kn; top > 0;) {
-                    const uint32_t k0 = top > kSolveBatch ? top - kSolveBatch : 0;
-                    Cf r[kSolveBatch];
-                    load_batch(r, row, k0, top, w);
-#pragma unroll
-                    for (uint32_t q = kSolveBatch; q-- > 0;)
-                        if (k0 + q < top && ((w >> (k0 + q)) & 1u)) xi = sgb_fma(-(V)r[q], x[kb + k0 + q], xi);
-                    top = k0;
-                }
-                x[i] = xi;
-            }
-            sync();
-        }
-    }
-
     // Mixed: out = W^-1 rb by the FP32 LU, then `sweeps` FP64-residual refinement sweeps.
     __device__ void solve_refined(const DevArgs &A, double ghinv, double *out) {
         float *xs = x32;
@@ -677,7 +894,9 @@ struct CoopCell {
         for (uint32_t sw = 0; sw < A.ir_sweeps; ++sw) {
             for (uint32_t i = tid; i < n; i += NT) {
                 double w = ghinv * out[i];
-                for (uint32_t e = tb.jrow[i]; e < tb.jrow[i + 1]; ++e) w = sgb_fma(js[e], out[tb.jcol[e]], w);
+                const uint32_t end = tb.jrow[i + 1];
+#pragma unroll 8
+                for (uint32_t e = tb.jrow[i]; e < end; ++e) w = sgb_fma(js[e], out[tb.jcol[e]], w);
                 xs[i] = (float)(rb[i] - w);
             }
             sync();
@@ -765,6 +984,7 @@ struct CoopCell {
         sync();
         if (tid == 0) {   // error norm and step factor once, shared through red[0..1]
             double e = 0.0;
+#pragma unroll 8
             for (uint32_t s = 0; s < n; ++s) e = sgb_fma(qv[s], qv[s], e);
             e = vsqrt(e * inv_n);
             if (!is_finite_lane(e)) e = 1e10;
@@ -810,7 +1030,7 @@ __global__ void __launch_bounds__(512, 1) kin_coop_kernel(const __grid_constant_
     extern __shared__ __align__(16) double sm[];
     __shared__ uint32_t cell_s;
     CoopCell<PREC> C;
-    C.tb.init(A.tables);
+    C.tb.init((const CoopMech *)A.tables, (const unsigned char *)A.tables);
     C.n = C.tb.h->n;
     C.R = C.tb.h->R;
     C.ld = C.tb.h->ld;
@@ -826,12 +1046,12 @@ __global__ void __launch_bounds__(512, 1) kin_coop_kernel(const __grid_constant_
     C.qv = C.ytmp + n;
     C.rb = C.qv + n;
     C.xv = C.rb + n;
-    C.y = C.xv + n;
+    C.rate = C.xv + n;   // the products of a Jacobian take everything up to here and the rates
+    C.y = C.rate + C.R;
     C.fcn = C.y + n;
     C.src = C.fcn + n;
     C.kr = C.src + n;
-    C.rate = C.kr + C.R;
-    C.red = C.rate + C.R;
+    C.red = C.kr + C.R;
     C.x32 = (float *)(sm + coop_smem_doubles(n, C.R));
     uint32_t *pat_s = (uint32_t *)(C.x32 + kCoopMaxSpecies);
     uint16_t *lcnt_s = (uint16_t *)(pat_s + (size_t)n * 8);
@@ -853,6 +1073,7 @@ __global__ void __launch_bounds__(512, 1) kin_coop_kernel(const __grid_constant_
         C.a = lay.lu_bytes ? (typename CoopCell<PREC>::Cf *)(smb + lay.lu) : (typename CoopCell<PREC>::Cf *)g;
         C.js = nullptr;
     }
+    C.prod = coop_products_fit(*C.tb.h) ? C.K : g + coop_scratch_base(PREC, *C.tb.h);
 #ifndef SGB_COOP_LOADS_FIRST_SMEM
 #define SGB_COOP_LOADS_FIRST_SMEM 0
 #endif
@@ -862,15 +1083,7 @@ __global__ void __launch_bounds__(512, 1) kin_coop_kernel(const __grid_constant_
         const uint4 *src = (const uint4 *)((const unsigned char *)A.tables + h->off_reac);
         uint4 *dst = (uint4 *)(smb + lay.terms);
         for (uint32_t q = threadIdx.x; q < lay.terms_bytes / 16; q += blockDim.x) dst[q] = src[q];
-        unsigned char *t = smb + lay.terms - h->off_reac;   // image offset o lives at t + o
-        C.tb.reac = (const uint16_t *)(t + h->off_reac);
-        C.tb.fbeg = (const uint32_t *)(t + h->off_fbeg);
-        C.tb.fent = (const CoopTerm *)(t + h->off_fent);
-        C.tb.jbeg = (const uint32_t *)(t + h->off_jbeg);
-        C.tb.jent = (const CoopTerm *)(t + h->off_jent);
-        C.tb.jpos = (const uint32_t *)(t + h->off_jpos);
-        C.tb.jrow = (const uint32_t *)(t + h->off_jrow);
-        C.tb.jcol = (const uint16_t *)(t + h->off_jcol);
+        C.tb.init(h, smb + lay.terms - h->off_reac);   // image offset o lives at terms - off_reac + o
     }
     __syncthreads();
     for (;;) {
@@ -927,7 +1140,7 @@ size_t coop_smem_bytes(int prec, const CoopMech &h, uint32_t budget = kCoopSmemB
 }
 
 size_t coop_scratch_doubles(int prec, const CoopMech &h) {
-    size_t d = prec == 2 ? (size_t)h.nj : (size_t)h.n * h.ld;
+    const size_t d = coop_scratch_base(prec, h) + (coop_products_fit(h) ? 0u : h.pairs);
     return (d + 31) / 32 * 32;   // 256-byte aligned per CTA
 }
 
