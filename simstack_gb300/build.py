@@ -84,7 +84,7 @@ def build(force: bool = False, jobs: int | None = None) -> str:
         ("kern_table_p1.o", [NVCC, *NV_FLAGS, "-DSGB_PREC=1", "-c", os.path.join(CSRC, "kern_table.cu")]),
         ("kern_table_p2.o", [NVCC, *NV_FLAGS, "-DSGB_PREC=2", "-c", os.path.join(CSRC, "kern_table.cu")]),
         *[(f"kern_group_p{p}_{n}.o", [NVCC, *NV_FLAGS, f"-DSGB_PREC={p}", f"-DSGB_NM={n}", "-c", os.path.join(CSRC, "kern_group.cu")])
-          for p in (4, 0, 1) for n in (32, 20, 12)],
+          for p in (4, 0, 1) for n in (32, 20, 17, 12)],
         ("kern_probe.o", [NVCC, *NV_FLAGS, "-c", os.path.join(CSRC, "kern_probe.cu")]),
         ("gpu_module.o", [NVCC, *NV_FLAGS, "-c", os.path.join(CSRC, "gpu_module.cu")]),
         ("static_scratch.o", [NVCC, *NV_FLAGS, "-c", os.path.join(CSRC, "static_scratch.cu")]),

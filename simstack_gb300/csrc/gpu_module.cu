@@ -272,7 +272,7 @@ cudaError_t launch_advance(uint32_t prec, const AdvanceShape &s, const DevArgs &
     if (e != cudaSuccess) return e;
     A.resume = 1;
     A.cursor = g.d_cursor;
-    return launch_group(prec, 0, A, g.stream);
+    return launch_group(prec, prec == 0 ? 0 : 1, A, g.stream);   // mixed CTAs park few: 16 lanes per cell
 }
 
 // The lane kernels (one cell per thread) for `A`, on `stream` (default: the module stream); the

@@ -12,15 +12,20 @@ typedef void (*GroupFn)(DevArgs, GroupArgs);
 // The kernel of a lane precision for mechanisms of at most NM species (kern_group.cu).
 template <int PREC, int NM> GroupFn group_kernel(uint32_t G, bool rodas3);
 template <> GroupFn group_kernel<0, 12>(uint32_t, bool);
+template <> GroupFn group_kernel<0, 17>(uint32_t, bool);
 template <> GroupFn group_kernel<0, 20>(uint32_t, bool);
 template <> GroupFn group_kernel<0, 32>(uint32_t, bool);
 template <> GroupFn group_kernel<1, 12>(uint32_t, bool);
+template <> GroupFn group_kernel<1, 17>(uint32_t, bool);
 template <> GroupFn group_kernel<1, 20>(uint32_t, bool);
 template <> GroupFn group_kernel<1, 32>(uint32_t, bool);
 template <> GroupFn group_kernel<4, 12>(uint32_t, bool);
+template <> GroupFn group_kernel<4, 17>(uint32_t, bool);
 template <> GroupFn group_kernel<4, 20>(uint32_t, bool);
 template <> GroupFn group_kernel<4, 32>(uint32_t, bool);
 template <int PREC> GroupFn group_kernel_for(uint32_t n, uint32_t G, bool rodas3) {
+    // FP64 at 8 lanes is faster without (4,096 cells x 1 s: 23.2 against 24.6 ms)
+    if (n == kGroupExact && rodas3 && !(PREC == 0 && G == 8)) return group_kernel<PREC, (int)kGroupExact>(G, true);
     return n <= 12 ? group_kernel<PREC, 12>(G, rodas3) : n <= 20 ? group_kernel<PREC, 20>(G, rodas3) : group_kernel<PREC, 32>(G, rodas3);
 }
 
@@ -44,7 +49,7 @@ inline int group_rule(uint32_t lane_prec, bool generated, uint32_t n, uint32_t l
     const uint32_t c = (lanes + (uint32_t)sms - 1) / (uint32_t)sms;
     if (lane_prec != 0 && lane_prec != 1 && lane_prec != 4) return -1;   // the other mixed variants: lanes only
     if (generated && lane_prec == 1) return -1;   // f32 lanes are as fast from one zone on (64 zones pulsed: 20.6 against 22.2)
-    if (c <= (lane_prec == 4 ? 10u : 8u)) return 2;
+    if (c <= (generated ? (lane_prec == 4 ? 10u : 8u) : (lane_prec == 4 ? 8u : 11u))) return 2;
     if (c <= (lane_prec == 4 ? 26u : 16u)) return 1;
     if (generated) return c <= (lane_prec == 4 ? 42u : 78u) ? 0 : -1;
     return lane_prec != 0 || c <= (n > 24 ? 128u : 400u) ? 0 : -1;

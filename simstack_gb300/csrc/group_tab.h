@@ -46,6 +46,9 @@ struct GroupHead {
 };
 static_assert(sizeof(GroupHead) % 16 == 0, "image alignment");
 constexpr uint32_t kGroupNone = 0xffffu;
+// The size of the shipped mechanism, which has kernels of its own with n a constant (any mechanism of that
+// many species under Rodas3 runs them).
+constexpr uint32_t kGroupExact = 17;
 // term words: the byte offset of the rate or product in bits 0..15, the coefficient's top 16
 // bits as a double (FP64 image) or a float (FP32 images) in bits 16..31
 constexpr uint32_t kGroupNoReactant = 0x8000u;   // RHS terms: bit 15, a reaction without reactants

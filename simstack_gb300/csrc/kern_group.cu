@@ -8,7 +8,7 @@
 #include "kin_group.cuh"
 
 #if !defined(SGB_PREC) || !defined(SGB_NM)
-#error "compile with -DSGB_PREC=0, 1 or 4 and -DSGB_NM=12, 20 or 32"
+#error "compile with -DSGB_PREC=0, 1 or 4 and -DSGB_NM=12, 17, 20 or 32"
 #endif
 
 namespace sgb {
@@ -21,7 +21,12 @@ template <class M> GroupFn of_lanes(uint32_t G) {
 }   // namespace
 
 template <> GroupFn group_kernel<SGB_PREC, SGB_NM>(uint32_t G, bool rodas3) {
+#if SGB_NM == 17   // exact n: Rodas3 only (group_kernel_for)
+    (void)rodas3;
+    return of_lanes<Rodas3Coef>(G);
+#else
     return rodas3 ? of_lanes<Rodas3Coef>(G) : of_lanes<RuntimeCoef>(G);
+#endif
 }
 
 }   // namespace sgb
