@@ -204,16 +204,6 @@ AdvanceShape shape_for(uint32_t prec, uint32_t lanes, bool with_mode) {
 // CTA queue kernel (FP64 and the default mixed variant).
 bool handoff(uint32_t prec) { return g.straggler_budget && g.group.dev && (lane_prec(prec) == 0 || lane_prec(prec) == 4); }
 
-// Cells at which a CTA of the queue kernel parks what it has left: where its attempt costs what a
-// group kernel takes for as many cells at full throughput. Shipped mechanism, cycles: FP64 lanes
-// 308k per 128-lane attempt against ~9.3k per cell and attempt of 8-lane groups (33 cells), mixed
-// 149k per 256 lanes against ~6.5k (23); the table lanes take ~2M per 128, so any CTA that is not full parks.
-uint32_t drain_at(uint32_t prec, const GpuKinTuning &t) {
-    if (t.kind != 2) return 0;
-    if (!g.generated) return t.block - 1;
-    return lane_prec(prec) == 0 ? t.block / 4 : t.block / 11;
-}
-
 // The group kernel on cells of `A` (its cursor is zeroed first), or on the parked ones (A.resume).
 cudaError_t launch_group(uint32_t prec, int group, const DevArgs &A0, cudaStream_t stream) {
     DevArgs A = A0;
@@ -263,7 +253,7 @@ cudaError_t launch_advance(uint32_t prec, const AdvanceShape &s, const DevArgs &
     if (!handoff(prec)) return launch_lanes(prec, t, A0);
     DevArgs A = A0;
     A.budget = prec == 0 ? g.straggler_budget : 0;
-    A.drain = drain_at(prec, t);
+    A.drain = t.kind == 2 ? group_drain(lane_prec(prec), g.generated, t.block) : 0;
     A.suspend_cap = kSuspendCap;
     A.suspend_count = g.d_suspend_count;
     A.suspend = g.d_suspend;

@@ -55,6 +55,15 @@ inline int group_rule(uint32_t lane_prec, bool generated, uint32_t n, uint32_t l
     return lane_prec != 0 || c <= (n > 24 ? 128u : 400u) ? 0 : -1;
 }
 
+// Cells at which a CTA of `block` lanes of the queue kernel parks what it has left: where its attempt costs
+// what a group kernel takes for as many cells at full throughput. Shipped mechanism, cycles: FP64 lanes
+// 308k per 128-lane attempt against ~9.3k per cell and attempt of 8-lane groups (33 cells), mixed
+// 149k per 256 lanes against ~6.5k (23); the table lanes take ~2M per 128, so any CTA that is not full parks.
+inline uint32_t group_drain(uint32_t lane_prec, bool generated, uint32_t block) {
+    if (!generated) return block - 1;
+    return lane_prec == 0 ? block / 4 : block / 11;
+}
+
 // One mechanism's schedule images on the device: per lanes-per-cell and lane precision (0 FP64, 1 f32
 // Delta, 2 mixed). Empty (dev null) for a mechanism whose record could not be laid out.
 struct GroupSet {

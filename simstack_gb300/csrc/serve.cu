@@ -154,7 +154,8 @@ struct Request {
     uint64_t footprint = 0;     // device bytes while running
     double *d_block = nullptr;  // zone block [rows][padded]
     double *d_inlet = nullptr;  // [n] inlet state
-    unsigned char *d_scratch = nullptr;   // queue cursor (+0), error flag (+128), table image (+256)
+    unsigned char *d_scratch = nullptr;   // queue cursor (+0), hand-off count (+64) and cursor (+68), error flag (+128), table image (+256)
+    SuspendRec *d_suspend = nullptr;      // cells the lane kernel's CTAs hand to a group kernel
     double *d_coop = nullptr;             // cooperative mechanism: per-CTA LU / Jacobian scratch
     uint32_t coop_grid = 0;
     cudaStream_t stream = nullptr;
@@ -222,6 +223,7 @@ void release(Request *r) {
         if (r->d_inlet) cudaFreeAsync(r->d_inlet, r->stream);
         if (r->d_scratch) cudaFreeAsync(r->d_scratch, r->stream);
         if (r->d_coop) cudaFreeAsync(r->d_coop, r->stream);
+        if (r->d_suspend) cudaFreeAsync(r->d_suspend, r->stream);
         cudaStreamDestroy(r->stream);
     }
     if (r->step_done) cudaEventDestroy(r->step_done);
@@ -231,6 +233,7 @@ void release(Request *r) {
     r->d_block = r->d_inlet = nullptr;
     r->d_scratch = nullptr;
     r->d_coop = nullptr;
+    r->d_suspend = nullptr;
 }
 
 // Allocates and uploads an admitted request, then captures its coupling step.
@@ -346,6 +349,25 @@ cudaError_t admit(Request *r) {
     const uint32_t resident = (uint32_t)per_sm * (uint32_t)E.sms, needed = (q.cells + sh.block - 1) / sh.block;
     sh.grid = resident < needed ? resident : needed;
 
+    // The lane kernel's CTAs park their last cells for a group kernel behind it (group_drain), as in a plain
+    // advance: at most grid * drain records, half a megabyte, which the footprint leaves out.
+    DevArgs resume = A;
+    int resume_group = -1;
+    if (group < 0 && gs.dev && (kp == 0 || kp == 4)) {
+        A.drain = group_drain(kp, r->generated, sh.block);
+        const uint32_t most = sh.grid * A.drain;
+        A.suspend_cap = most < q.cells ? most : q.cells;
+        e = cudaMallocAsync((void **)&r->d_suspend, A.suspend_cap * sizeof(SuspendRec), r->stream);
+        if (e != cudaSuccess) return e;
+        A.suspend = r->d_suspend;
+        A.suspend_count = (uint32_t *)(r->d_scratch + 64);
+        resume = A;
+        resume.resume = 1;
+        resume.cursor = (uint32_t *)(r->d_scratch + 68);
+        resume_group = group_rule(kp, r->generated, r->n, A.suspend_cap, E.sms);
+        if (resume_group < 0) resume_group = 0;
+    }
+
     // one launch with no lanes outside the capture: loads the kernel and sets
     // its attributes (it returns right after staging its tables)
     DevArgs idle = A;
@@ -354,14 +376,17 @@ cudaError_t admit(Request *r) {
         return group >= 0 ? gs.launch(kp, group, a, q.cells, E.sms, r->stream) : launch_chem(r->generated, kp, sh, a, r->stream);
     };
     e = chem(idle);
+    // (the resume kernel finds nothing parked: the count is zero)
+    if (e == cudaSuccess && resume_group >= 0) e = gs.launch(kp, resume_group, resume, A.suspend_cap, E.sms, r->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(r->stream);
     if (e != cudaSuccess) return e;
 
     cudaGraph_t graph = nullptr;
     e = cudaStreamBeginCapture(r->stream, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return e;
-    cudaError_t ce = cudaMemsetAsync(r->d_scratch, 0, sizeof(uint32_t), r->stream);   // the cursor; the error flag stays sticky
+    cudaError_t ce = cudaMemsetAsync(r->d_scratch, 0, 128, r->stream);   // cursors and count; the error flag stays sticky
     if (ce == cudaSuccess) ce = chem(A);
+    if (ce == cudaSuccess && resume_group >= 0) ce = gs.launch(kp, resume_group, resume, A.suspend_cap, E.sms, r->stream);
     if (ce == cudaSuccess)
         ce = (cudaError_t)gpu_advect(A.y, P, r->n, q.cells, q.channel_cells, r->d_inlet, r->courant, r->substeps, r->stream);
     e = cudaStreamEndCapture(r->stream, &graph);
