@@ -72,6 +72,7 @@ struct Module {
     uint64_t arena_size = 0, arena_used = 0;
     // mechanism
     bool have_mech = false, generated = false;
+    bool plans = false;            // the group and cooperative images are those of `mech`
     KinMech mech;
     KinMethod method;
     KinControl control;
@@ -385,6 +386,13 @@ SGB_API int32_t gpu_init(uint32_t device_index, uint64_t arena_bytes, GpuInfo *i
         if (g.d_dbd_scratch) cudaFree(g.d_dbd_scratch);
         g.d_dbd_scratch = nullptr;
         g.dbd_scratch_bytes = 0;
+        g.group.release();   // the mechanism's images and scratch, on the device they were made on
+        if (g.coop_image_buffer) cudaFree(g.coop_image_buffer);
+        if (g.d_coop_scratch) cudaFree(g.d_coop_scratch);
+        g.coop_image_buffer = g.d_coop_image = nullptr;
+        g.d_coop_scratch = nullptr;
+        g.coop_image_bytes = g.coop_scratch_bytes = 0;
+        g.plans = false;
         g.arena = nullptr;
         g.d_tables = nullptr;
         g.d_cursor = nullptr;
@@ -529,12 +537,17 @@ SGB_API int32_t gpu_kin_set_mech(const KinMech *mech, const KinMethod *method, c
     cudaError_t e = cudaMemcpyAsync(g.d_tables, image, kTableBytes, cudaMemcpyHostToDevice, g.stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(g.stream);
     if (e != cudaSuccess) return (int32_t)e;
+    // The group and cooperative images depend on the mechanism alone: the same record as before keeps them.
+    const bool same = g.plans && memcmp(&g.mech, mech, sizeof(KinMech)) == 0;
     g.mech = *mech;
     g.method = *method;
     g.control = *control;
     g.generated = fnv1a(mech, sizeof(KinMech)) == air_ops_signature() && method_is_rodas3(method);
     g.have_mech = true;
-    e = g.group.build(*mech, method_is_rodas3(method));
+    g.group.rodas3 = method_is_rodas3(method);
+    if (same) return 0;
+    g.plans = false;
+    e = g.group.build(*mech, g.group.rodas3);
     if (e != cudaSuccess) return (int32_t)e;
     // the cooperative image of the same mechanism (tuning kind 3, mode 1)
     // (the buffers are kept while they are large enough: the stream is idle here)
@@ -550,6 +563,7 @@ SGB_API int32_t gpu_kin_set_mech(const KinMech *mech, const KinMethod *method, c
         if (e != cudaSuccess) return (int32_t)e;
         g.d_coop_image = g.coop_image_buffer;
     }
+    g.plans = true;
     return 0;
 }
 
