@@ -415,7 +415,7 @@ struct CoopCell {
     // stage vectors K (multipliers) and the four vectors after them (U rows), free until the
     // stages begin, so B is 4 in FP64 and 8 in FP32; the pattern words use x32. Measured on 200 species /
     // 1,200 reactions, cycles per factorisation: FP64 one CTA per SM 3.05M -> 1.90M, two (per pair of
-    // cells) 2.77M of 2.5M that its FP64 instructions take at the unit's rate; FP32 550k -> 357k.
+    // cells) 2.62M, most of it FP64 instructions at the rate of their unit; FP32 550k -> 357k.
     template <uint32_t B>
     __device__ void factor_panels(Cf ghinv) {
         static_assert(B * sizeof(Cf) <= 32, "panel buffers: 32 bytes per row in K, and as much for the U rows");
@@ -498,6 +498,10 @@ struct CoopCell {
             }
             sync();
             for (uint32_t c = j0; c < n; c += 32) {
+                if (n - c <= 16) {   // the last columns: two or four rows to a warp
+                    trailing_rest<B>(Lp, Up, live, rows_on, c, j0, n - c <= 8 ? 8u : 16u);
+                    break;
+                }
                 const uint32_t jc = c + lane;
                 const bool on = jc < n;
                 const uint32_t lc = on ? live[jc] : 0u;
@@ -539,6 +543,40 @@ struct CoopCell {
             sync();
         }
         sync();
+    }
+
+    // The trailing update's last `width` (8 or 16) columns or fewer: a row's FMA there would use a quarter or half
+    // of the lanes for the FP64 unit's same 64 cycles, so a warp takes 32 / width rows side by side
+    // (200 species, two cells per SM: 2.77M -> 2.62M cycles per factorisation).
+    template <uint32_t B>
+    __device__ __forceinline__ void trailing_rest(const Cf *Lp, const Cf *Up, const uint16_t *live, const uint16_t *rows_on, uint32_t c,
+                                                  uint32_t j0, uint32_t width) {
+        const uint32_t jc = c + (lane & (width - 1)), rows = 32 / width, step = W * rows;
+        const uint32_t lc = jc < n ? live[jc] : 0u;
+        if (!__any_sync(0xffffffffu, lc != 0)) return;
+        Cf u[B];
+#pragma unroll
+        for (uint32_t p = 0; p < B; ++p) u[p] = jc < n ? Up[p * n + jc] : (Cf)0.0;
+        for (uint32_t i0 = j0 + warp * rows; i0 < n; i0 += 2 * step) {   // two rows per lane: their loads overlap
+            uint32_t m[2];
+            Cf v[2];
+#pragma unroll
+            for (uint32_t r = 0; r < 2; ++r) {
+                const uint32_t ii = i0 + lane / width + r * step;
+                m[r] = ii < n ? rows_on[ii] & lc : 0u;
+                v[r] = m[r] ? a[(size_t)ii * ld + jc] : (Cf)0.0;
+            }
+#pragma unroll
+            for (uint32_t r = 0; r < 2; ++r) {
+                const uint32_t ii = i0 + lane / width + r * step;
+                if (!m[r]) continue;
+                const Cf *lp = Lp + ii * B;
+#pragma unroll
+                for (uint32_t p = 0; p < B; ++p)
+                    if ((m[r] >> p) & 1u) v[r] = sgb_fma(-lp[p], u[p], v[r]);
+                a[(size_t)ii * ld + jc] = v[r];
+            }
+        }
     }
 
     // factor_panels in FP32, B = 8, without pattern tests: an element off the pattern is zero and stays
