@@ -6,17 +6,18 @@
 // (src/sim/kinetics/kin_solver.h:40-139) per element:
 //   - RHS: f[s] = src[s], then fma(net, rate_r, f[s]) over reactions r ascending;
 //   - Jacobian: a[slot] = 0, then fma(-net, d_rp, a[slot]) over (r, p, e) ascending;
-//   - LU: the elimination runs pivot by pivot (KIJ) instead of row by row
-//     (IKJ), which applies the same updates to every element in the same
-//     (ascending pivot) order, so the results are the same bits;
-//   - solves: in blocks of 32 columns (a warp solves the diagonal block, then
+//   - LU: the elimination runs in panels of pivots (or pivot by pivot, KIJ)
+//     instead of row by row (IKJ), which applies the same updates to every
+//     element in the same (ascending pivot) order, so the results are the same bits;
+//   - solves: in blocks of columns (a warp solves the diagonal block, then
 //     every row outside it takes the block's updates one by one), which gives
 //     every x[i] its updates in the reference's order (lower: ascending
 //     column; upper: descending column, then the diagonal).
 // The LU lives in a dense [n][ld] array (the filled pattern is 78-87% dense
 // for a 200-species random mechanism in natural order); the kernels walk it
-// densely and test each element against the pattern bitmask, so only
-// pattern elements are ever updated, as in the reference.
+// densely. The FP64 ones test each element against the pattern bitmask, so only
+// pattern elements are ever updated, as in the reference; the FP32 panels and solves
+// multiply by the zeros that stand off the pattern.
 #pragma once
 #include <stdint.h>
 
@@ -37,15 +38,8 @@ struct CoopMech {
     uint32_t bytes;           // image size
     // byte offsets from the image start (each 16-byte aligned)
     uint32_t off_reac;        // uint16[R][4]: reactant count, then up to 3 reactant species
-    uint32_t off_jpos;        // uint32[nj]: row * ld + col
     uint32_t off_jrow;        // uint32[n+1]: entries of row i are [jrow[i], jrow[i+1])
     uint32_t off_jcol;        // uint16[nj]
-    uint32_t off_lbeg;        // uint32[n+1]
-    uint32_t off_lrow;        // uint16[]: rows i > k with (i, k) in the filled pattern, per column k
-    uint32_t off_ubeg;        // uint32[n+1]
-    uint32_t off_ucol;        // uint16[]: columns j > k with (k, j) in the filled pattern, per row k
-    uint32_t off_cbeg;        // uint32[n+1]
-    uint32_t off_crow;        // uint16[]: rows i < k with (i, k) in the filled pattern, per column k
     uint32_t off_pat;         // uint32[n][8]: filled pattern, bit j of row i (n <= 256)
     uint32_t off_lcnt;        // uint16[n]: rows below the diagonal in column k
     uint32_t pairs;           // (reaction, reactant) pairs

@@ -131,32 +131,20 @@ bool build_image(const Desc &d, std::vector<uint8_t> *out) {
     }
     h.nj = (uint32_t)jpos.size();
     for (uint32_t i = 0; i < n; ++i) jrow[i + 1] += jrow[i];
-    // elimination lists
-    std::vector<uint32_t> lbeg(n + 1), ubeg(n + 1), cbeg(n + 1);
-    std::vector<uint16_t> lrow, ucol, crow;
-    for (uint32_t k = 0; k < n; ++k) {
-        lbeg[k] = (uint32_t)lrow.size();
-        ubeg[k] = (uint32_t)ucol.size();
-        cbeg[k] = (uint32_t)crow.size();
-        for (uint32_t i = k + 1; i < n; ++i)
-            if (pat_at(i, k)) lrow.push_back((uint16_t)i);
-        for (uint32_t j = k + 1; j < n; ++j)
-            if (pat_at(k, j)) ucol.push_back((uint16_t)j);
-        for (uint32_t i = 0; i < k; ++i)
-            if (pat_at(i, k)) crow.push_back((uint16_t)i);
-        h.lu_updates += (uint64_t)(lrow.size() - lbeg[k]) * (ucol.size() - ubeg[k]);
-    }
-    lbeg[n] = (uint32_t)lrow.size();
-    ubeg[n] = (uint32_t)ucol.size();
-    cbeg[n] = (uint32_t)crow.size();
     std::vector<uint32_t> pat((size_t)n * 8, 0u);
-    std::vector<uint16_t> lcnt(n, 0);
+    std::vector<uint16_t> lcnt(n, 0), ucnt(n, 0);
     for (uint32_t i = 0; i < n; ++i)
         for (uint32_t j = 0; j < n; ++j)
             if (pat_at(i, j)) {
                 pat[(size_t)i * 8 + (j >> 5)] |= 1u << (j & 31);
                 if (i > j) lcnt[j]++;
+                if (i < j) ucnt[i]++;
             }
+    for (uint32_t k = 0; k < n; ++k) {
+        h.l_entries += lcnt[k];
+        h.u_entries += ucnt[k];
+        h.lu_updates += (uint64_t)lcnt[k] * ucnt[k];
+    }
     // pairs and grouped lists
     std::vector<uint32_t> pair, fgrp, fdst, jgrp, jdst;
     std::vector<CoopWide> fterm, jterm;
@@ -221,8 +209,6 @@ bool build_image(const Desc &d, std::vector<uint8_t> *out) {
         group(jl, jt, &jgrp, &jdst, &jterm);
         if (!wide_ok) return false;   // a net change that is no small integer
     }
-    h.l_entries = (uint32_t)lrow.size();
-    h.u_entries = (uint32_t)ucol.size();
 
     // layout
     size_t off = align16(sizeof(CoopMech));
@@ -238,15 +224,8 @@ bool build_image(const Desc &d, std::vector<uint8_t> *out) {
     place(&h.off_jgrp, jgrp.size() * 4);
     place(&h.off_jdst, jdst.size() * 4);
     place(&h.off_jterm, jterm.size() * sizeof(CoopWide));
-    place(&h.off_jpos, jpos.size() * 4);
     place(&h.off_jrow, jrow.size() * 4);
     place(&h.off_jcol, jcol.size() * 2);
-    place(&h.off_lbeg, lbeg.size() * 4);
-    place(&h.off_lrow, lrow.size() * 2);
-    place(&h.off_ubeg, ubeg.size() * 4);
-    place(&h.off_ucol, ucol.size() * 2);
-    place(&h.off_cbeg, cbeg.size() * 4);
-    place(&h.off_crow, crow.size() * 2);
     place(&h.off_pat, pat.size() * 4);
     place(&h.off_lcnt, lcnt.size() * 2);
     if (off > 0xffffffffu) return false;
@@ -258,15 +237,8 @@ bool build_image(const Desc &d, std::vector<uint8_t> *out) {
         if (bytes) memcpy(b + o, src, bytes);
     };
     put(h.off_reac, reac.data(), reac.size() * 2);
-    put(h.off_jpos, jpos.data(), jpos.size() * 4);
     put(h.off_jrow, jrow.data(), jrow.size() * 4);
     put(h.off_jcol, jcol.data(), jcol.size() * 2);
-    put(h.off_lbeg, lbeg.data(), lbeg.size() * 4);
-    put(h.off_lrow, lrow.data(), lrow.size() * 2);
-    put(h.off_ubeg, ubeg.data(), ubeg.size() * 4);
-    put(h.off_ucol, ucol.data(), ucol.size() * 2);
-    put(h.off_cbeg, cbeg.data(), cbeg.size() * 4);
-    put(h.off_crow, crow.data(), crow.size() * 2);
     put(h.off_pat, pat.data(), pat.size() * 4);
     put(h.off_lcnt, lcnt.data(), lcnt.size() * 2);
     put(h.off_pair, pair.data(), pair.size() * 4);

@@ -1,8 +1,9 @@
 // Cooperative kernels for large mechanisms: one CTA integrates one cell at a
 // time (persistent CTAs take cells from a work queue), its threads splitting
-// every phase of the Rosenbrock step -- rates per reaction, RHS per species,
-// Jacobian per entry, elimination per (row, column) of each pivot (two pivots
-// per pass for an FP64 LU in global memory), solves per row of each column. The step control is the reference's
+// every phase of the Rosenbrock step -- rates per reaction, RHS and Jacobian
+// per species and entry from products formed once, elimination in panels of
+// four (FP64) or eight (FP32) pivots with a thread per row, solves with a thread per
+// row in blocks of columns. The step control is the reference's
 // (src/sim/kinetics/kin_solver.h:189-345): every thread runs the scalar
 // controller on the same values, so its decisions are uniform across the CTA.
 //
@@ -85,7 +86,7 @@ constexpr uint32_t kCoopSmemBudget = 0;
 
 // Shared memory of one CTA: doubles, x32 (256 floats), pattern (n x 8 words), lcnt (n u16,
 // padded), then the LU (mixed always, n x ld floats; FP64 when it fits kCoopSmemLuF64Max), then
-// -- when they fit the budget -- the RHS / Jacobian term lists (image bytes [off_reac, off_lbeg)).
+// -- when they fit the budget -- the RHS / Jacobian term lists (image bytes [off_reac, off_pat)).
 struct CoopSmemLayout {
     size_t lu, lu_bytes, terms, terms_bytes, total;
 };
@@ -95,7 +96,7 @@ __host__ __device__ inline CoopSmemLayout coop_layout(int prec, const CoopMech &
     const size_t lu64 = (size_t)h.n * h.ld * sizeof(double);
     L.lu_bytes = prec == 2 ? (size_t)h.n * h.ld * 4 : (lu64 <= kCoopSmemLuF64Max ? lu64 : 0);
     L.terms = (L.lu + L.lu_bytes + 15) / 16 * 16;
-    const size_t tb = (size_t)h.off_lbeg - h.off_reac;
+    const size_t tb = (size_t)h.off_pat - h.off_reac;
     L.terms_bytes = L.terms + tb <= budget ? tb : 0;
     L.total = L.terms + L.terms_bytes;
     return L;
@@ -1112,10 +1113,7 @@ __global__ void __launch_bounds__(512, 1) kin_coop_kernel(const __grid_constant_
         C.js = nullptr;
     }
     C.prod = coop_products_fit(*C.tb.h) ? C.K : g + coop_scratch_base(PREC, *C.tb.h);
-#ifndef SGB_COOP_LOADS_FIRST_SMEM
-#define SGB_COOP_LOADS_FIRST_SMEM 0
-#endif
-    C.lu_global = (PREC == 0 && lay.lu_bytes == 0) || (SGB_COOP_LOADS_FIRST_SMEM && n >= 64);
+    C.lu_global = PREC == 0 && lay.lu_bytes == 0;
     if (lay.terms_bytes) {   // the RHS / Jacobian term lists, once per CTA
         const CoopMech *h = C.tb.h;
         const uint4 *src = (const uint4 *)((const unsigned char *)A.tables + h->off_reac);
