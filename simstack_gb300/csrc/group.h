@@ -86,14 +86,16 @@ struct GroupSet {
                 all.insert(all.end(), one.begin(), one.end());
             }
         rodas3 = method_rodas3;
-        cudaError_t e = cudaSuccess;
         if (all.size() * 4 > capacity) {
             release();
-            e = cudaMalloc((void **)&buffer, all.size() * 4);
-            if (e != cudaSuccess) return e;
+            if (cudaMalloc((void **)&buffer, all.size() * 4) != cudaSuccess) {   // no memory: the lane kernels run alone
+                cudaGetLastError();
+                buffer = nullptr;
+                return cudaSuccess;
+            }
             capacity = all.size() * 4;
         }
-        e = cudaMemcpy(buffer, all.data(), all.size() * 4, cudaMemcpyHostToDevice);
+        const cudaError_t e = cudaMemcpy(buffer, all.data(), all.size() * 4, cudaMemcpyHostToDevice);
         if (e == cudaSuccess) dev = buffer;
         return e;
     }
