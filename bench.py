@@ -645,7 +645,7 @@ def run_ours(args):
 # measured on the oracle (64-cell sample, seed 3).
 UNEVEN_SOURCE_P0 = 1e-2
 # Straggler hand-off budget (FP64): cells past this many step attempts in one advance (about the p99
-# of this workload's step counts) finish on the cooperative kernel; the module's default.
+# of this workload's step counts) finish on a lane-group kernel; the module's default.
 UNEVEN_HANDOFF_BUDGET = 600
 
 
@@ -666,7 +666,7 @@ def run_uneven_stiffness(args):
     zf = None
     for prec in (0, 2):
         launch.precision = prec
-        for kind, budget in ((0, 0), (2, 0), (2, UNEVEN_HANDOFF_BUDGET)) if prec == 0 else ((0, 0), (2, 0)):
+        for kind, budget in ((0, 0), (2, 0), (2, UNEVEN_HANDOFF_BUDGET)):
             mod.set_straggler_budget(budget)
             sg.check(L.gpu_copy_on_device(work, pristine, z.nbytes), "copy")
             t = mod.autotune(launch, kind=kind)
@@ -718,7 +718,8 @@ def run_uneven_stiffness(args):
             "kernels": results,
             "queue_speedup_vs_static": {"f64": results["f64_static"]["ms"] / results["f64_queue"]["ms"],
                                         "mixed": results["mixed_static"]["ms"] / results["mixed_queue"]["ms"]},
-            "handoff_speedup_vs_static": {"f64": results["f64_static"]["ms"] / results["f64_queue_handoff"]["ms"]},
+            "handoff_speedup_vs_static": {p: results[f"{p}_static"]["ms"] / results[f"{p}_queue_handoff"]["ms"]
+                                          for p in ("f64", "mixed")},
             "roofline": {"bound": "fp32", "unit": "TFLOP/s", "peak": fp32_peak,
                          "achieved": MIXED_FP32_FLOPS_PER_CELL_STEP * attempts / (results[best]["ms"] * 1e-3) / 1e12,
                          "frac": MIXED_FP32_FLOPS_PER_CELL_STEP * attempts / (results[best]["ms"] * 1e-3) / 1e12 / fp32_peak,

@@ -217,7 +217,8 @@ SGB_API int32_t gpu_kin_advance_pipelined(const GpuKinLaunch *launch, void *host
  * gpu_kin_autotune times the candidates of `kind` on the given launch (which
  * it advances repeatedly on a scratch copy it restores) and keeps the fastest;
  * kind 4 times kinds 2 and 3 together, so the cells-per-warp decomposition is
- * chosen by measurement as well. */
+ * chosen by measurement as well. Where a lane-group kernel beats every candidate of kind 2 or 4,
+ * `best` is the fastest candidate and the module goes on choosing by batch size. */
 typedef struct GpuKinTuning {
     uint32_t kind, block, chunk, variant;
     float ms;
@@ -389,8 +390,8 @@ SGB_API int32_t gpu_advect(double *y, uint32_t padded, uint32_t species, uint32_
                            const double *inlet_device, double courant, uint32_t substeps, void *stream);
 
 /* Serving. A request is a block of cells integrated over `coupling_steps`
- * steps of `dt` seconds; every step is chemistry over dt (persistent queue
- * kernel), then film advection (operator split in the order of
+ * steps of `dt` seconds; every step is chemistry over dt (lane or lane-group
+ * kernels by the cells of all requests at hand), then film advection (operator split in the order of
  * src/sim/dbd_scene.cpp:263-265), captured once per request as a CUDA graph
  * and replayed on the request's own stream. Substeps follow the Courant-0.9
  * rule of src/sim/nft.cpp:531-536: ceil(dt / (0.9 dx / v)). The inlet of every
@@ -512,7 +513,7 @@ SGB_API void kin_model_counts(const KinModelHandle *model, uint64_t *counts);
 /* Reference-layout tables; cudaErrorInvalidValue (1) if the mechanism exceeds them. */
 SGB_API int32_t kin_model_kinmech(const KinModelHandle *model, KinMech *out);
 SGB_API uint64_t kin_mech_signature(const KinMech *mech); /* FNV-1a over the record */
-/* The cooperative kernels' wide-index image (pattern bitmask, term lists, elimination lists) of a
+/* The cooperative kernels' wide-index image (pattern bitmask, term lists) of a
  * finalized model or of a KinMech; returns its size (0 if it cannot be built) and copies it to
  * `out` when `capacity` suffices. The same mechanism gives the same bytes from either source. */
 SGB_API uint64_t kin_model_coop_image(const KinModelHandle *model, void *out, uint64_t capacity);

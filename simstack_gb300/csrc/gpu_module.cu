@@ -807,6 +807,7 @@ SGB_API int32_t gpu_kin_autotune(const GpuKinLaunch *launch, uint32_t kind, GpuK
     if (kind == 3 || kind == 4) list.insert(list.end(), std::begin(coop_cands), std::end(coop_cands));
     GpuKinTuning winner = g.tuning[launch->precision];
     winner.ms = 1e30f;
+    const bool was_tuned = g.tuned[launch->precision];
     // candidates that would grow the context's stack reservation are skipped, unless none fits
     size_t have = 0, least = (size_t)-1;
     cudaDeviceGetLimit(&have, cudaLimitStackSize);
@@ -833,11 +834,24 @@ SGB_API int32_t gpu_kin_autotune(const GpuKinLaunch *launch, uint32_t kind, GpuK
             winner.ms = best_ms;
         }
     }
+    // kinds 2 and 4: against what the batch size alone would choose, where that is a group kernel (4,096
+    // cells x 1 s: FP64 23.9 ms against 42.5 for the best lane candidate, mixed 14.7 against 20.8)
+    bool by_size = false;
+    g.tuned[launch->precision] = false;
+    const AdvanceShape untuned = shape_for(launch->precision, launch->lane_count ? launch->lane_count : launch->padded, true);
+    if ((kind == 2 || kind == 4) && untuned.group >= 0)
+        for (int rep = 0; rep < 2 && e == cudaSuccess; ++rep) {
+            float ms = 0.0f;
+            e = advance_sync(launch, nullptr, &ms);
+            copy_all(false);
+            by_size = by_size || ms < winner.ms;
+        }
     cudaStreamSynchronize(g.stream);
     cudaFree(save);
+    g.tuned[launch->precision] = was_tuned;
     if (e != cudaSuccess) return (int32_t)e;
-    g.tuning[launch->precision] = winner;
-    g.tuned[launch->precision] = true;
+    if (!by_size || winner.kind != 3) g.tuning[launch->precision] = winner;   // by size: the lane kernels' shape
+    g.tuned[launch->precision] = !by_size;
     if (best) *best = winner;
     return 0;
 }

@@ -128,3 +128,21 @@ def test_large_batches_by_rule(untuned, cells, precision):
     untuned.set_straggler_budget(sg.DEFAULT_STRAGGLER_BUDGET)
     sg.check(sg.lib().gpu_init(0, 2 << 30, untuned.info), "gpu_init")   # untuned again
     assert_bits(z, ref)
+
+
+@pytest.mark.parametrize("precision,kind,cells", [(0, 2, 700), (2, 4, 700), (0, 2, 16001)])
+def test_autotune_against_the_rule(untuned, oracle_lib, precision, kind, cells):
+    """An autotuned small batch keeps the rule's group kernel (no lane shape is near it), a large one takes the
+    measured lane shape; the same bits."""
+    untuned.set_mech(sg.Model.air().kinmech(), sg.method("rodas3"), sg.control())
+    z = sg.air_cells(cells, seed=9)
+    ref = z.copy()
+    base = untuned.upload(z)
+    t = untuned.autotune(z.launch(base, precision, 0.2), kind=kind)
+    ms = untuned.advance(z.launch(base, precision, 0.2))
+    if cells == 700:
+        assert ms < t.ms
+    untuned.download(z, base)
+    sg.check(sg.lib().gpu_init(0, 2 << 30, untuned.info), "gpu_init")   # untuned again
+    oracle_advance(oracle_lib, ref, 0.2, precision)
+    assert_bits(z, ref)
