@@ -13,8 +13,10 @@
 //
 // Coupling step (operator split, chemistry first, as dbd_scene.cpp:263-265):
 // [cursor reset] -> [chemistry over the request's zone block, 1 s: the
-// persistent queue kernel for the shipped or a KinMech table mechanism, the
-// cooperative one-CTA-per-cell kernel for a large mechanism] -> [advection].
+// lane-group kernel or, where the requests at hand fill the GPU, the persistent
+// queue kernel and a group kernel for the cells it parks (the shipped or a KinMech
+// table mechanism); the cooperative one-CTA-per-cell kernel for a large
+// mechanism] -> [advection].
 // Captured once per request into a CUDA graph and replayed every step on the
 // request's own stream; each request has its own queue scratch, so requests
 // run side by side.
@@ -354,18 +356,22 @@ cudaError_t admit(Request *r) {
     DevArgs resume = A;
     int resume_group = -1;
     if (group < 0 && gs.dev && (kp == 0 || kp == 4)) {
-        A.drain = group_drain(kp, r->generated, sh.block);
-        const uint32_t most = sh.grid * A.drain;
-        A.suspend_cap = most < q.cells ? most : q.cells;
-        e = cudaMallocAsync((void **)&r->d_suspend, A.suspend_cap * sizeof(SuspendRec), r->stream);
-        if (e != cudaSuccess) return e;
-        A.suspend = r->d_suspend;
-        A.suspend_count = (uint32_t *)(r->d_scratch + 64);
-        resume = A;
-        resume.resume = 1;
-        resume.cursor = (uint32_t *)(r->d_scratch + 68);
-        resume_group = group_rule(kp, r->generated, r->n, A.suspend_cap, E.sms);
-        if (resume_group < 0) resume_group = 0;
+        const uint32_t drain = group_drain(kp, r->generated, sh.block), most = sh.grid * drain;
+        const uint32_t cap = most < q.cells ? most : q.cells;
+        if (cudaMallocAsync((void **)&r->d_suspend, cap * sizeof(SuspendRec), r->stream) == cudaSuccess) {
+            A.drain = drain;
+            A.suspend_cap = cap;
+            A.suspend = r->d_suspend;
+            A.suspend_count = (uint32_t *)(r->d_scratch + 64);
+            resume = A;
+            resume.resume = 1;
+            resume.cursor = (uint32_t *)(r->d_scratch + 68);
+            resume_group = group_rule(kp, r->generated, r->n, cap, E.sms);
+            if (resume_group < 0) resume_group = 0;
+        } else {   // no memory left for the records: the lanes finish their cells themselves
+            cudaGetLastError();
+            r->d_suspend = nullptr;
+        }
     }
 
     // one launch with no lanes outside the capture: loads the kernel and sets
