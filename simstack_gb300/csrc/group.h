@@ -133,8 +133,14 @@ struct GroupSet {
                                           : lane_prec == 1 ? group_kernel_for<1>(n, G, rodas3) : group_kernel_for<4>(n, G, rodas3);
         const GroupArgs a = args(lane_prec, g);
         const uint32_t need = (want + 32 / G - 1) / (32 / G);   // warps
-        // few cells: one warp per CTA, so that they spread over the SMs; else one warp per scheduler and CTA
-        uint32_t warps = need <= (uint32_t)sms ? 1u : need <= 2u * (uint32_t)sms ? 2u : 4u;
+        const uint32_t each = (need + (uint32_t)sms - 1) / (uint32_t)sms;   // warps per SM, evenly spread
+        // FP64: one CTA per SM with just its share of warps up to 8. The FP64 unit is busy with four, so an SM
+        // with two CTAs of four where others have one takes twice as long (1 s of the shipped mechanism, 4,096 cells: 256
+        // CTAs on 152 SMs; 0.3 s, CTAs of four / of the share: 1,501 cells 14.8 / 13.2 ms, 3,000 21.2 / 19.1,
+        // 4,096 21.3 / 20.5; 24 species, 0.05 s, 2,400 cells 30.8 / 20.1). Else, as the mixed lanes
+        // wait for their chains and not for the unit (2,000 cells 9.0 / 9.3): few cells one or two warps per CTA,
+        // so that they spread over the SMs, and from there one warp per scheduler and CTA.
+        uint32_t warps = lane_prec == 0 && each <= 8 ? each : each <= 2 ? each : 4u;
         while (warps > 1 && smem(a, g, warps) > kSmemMax) --warps;
         const size_t bytes = smem(a, g, warps);
         cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);

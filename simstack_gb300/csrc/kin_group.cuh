@@ -1092,7 +1092,7 @@ constexpr uint32_t kGroupStateBytes = KIN_MAX_SPECIES * 8;
 // stops claiming, so that it gets there soon, and when there are fewer cells than warps each
 // warp claims one only.
 template <class M, int PREC, int G, int NM>
-__global__ void __launch_bounds__(128, 1) kin_group_kernel(const __grid_constant__ DevArgs A, const __grid_constant__ GroupArgs S) {
+__global__ void __launch_bounds__(PREC == 0 ? 256 : 128, 1) kin_group_kernel(const __grid_constant__ DevArgs A, const __grid_constant__ GroupArgs S) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) uint64_t bar;
     constexpr uint32_t kCells = 32 / G;

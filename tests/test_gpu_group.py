@@ -30,7 +30,8 @@ def oracle_advance(O, z, duration, precision, method="rodas3", ctl=None, mech=No
 
 # cells: one, a few, 32 lanes per cell (<= 8 or 10 per SM), 16 (<= 16 or 26), 8 (<= 96 or 48), and one lane
 @pytest.mark.parametrize("precision", [0, 2])
-@pytest.mark.parametrize("cells", [1, 3, 613, 1601, 2801, 5003])
+# (FP64: CTAs of 1, 1, 5, 6, 5, 8 and 4 warps)
+@pytest.mark.parametrize("cells", [1, 3, 613, 1601, 2801, 4801, 5003])
 def test_shipped_mechanism_by_size(untuned, oracle_lib, cells, precision):
     untuned.set_mech(sg.Model.air().kinmech(), sg.method("rodas3"), sg.control())
     z = sg.air_cells(cells, seed=cells)
