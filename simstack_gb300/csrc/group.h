@@ -41,6 +41,9 @@ constexpr uint32_t kGroupLanes[3] = {8, 16, 32};
 //                    8,192 cells: FP64 62.7 / 44.3 / 35.4 / 59.4   mixed 33.0 / 26.5 / 23.9 / 24.8
 //                   10,240 cells: FP64 8 lanes 41.7, lane kernel with its hand-off 46.6; 14,336: 52.2, 45.6
 //                    6,144 cells: mixed 8 lanes 21.2, lane kernel with its hand-off 21.9; 7,168: 22.8, 21.7
+// (in CTAs of four warps; launch() below now takes FP64's shape by the share, which moves 16 lanes forward:)
+//   table FP64, 0.05 s, 1,230 cells (9 per SM), 32 / 16 lanes: 16 species 14.2 / 11.4, 24 species
+//                    19.7 / 17.3, 32 species (0.02 s) 26.7 / 22.9; 1,660 cells 15.6 / 11.9, 20.8 / 17.8, 28.8 / 24.7
 // The table-driven lane kernels keep a cell's arrays in local memory (~1 ms per attempt) and win only
 // where they fill the GPU several times over (0.1 s, 65,536 cells, 8 lanes / lane kernel): FP64 8 species
 // 54 / 51, 16 species 176 / 203, 24 species 513 / 576, 32 species 16,384 cells 339 / 372 and 65,536
@@ -49,7 +52,7 @@ inline int group_rule(uint32_t lane_prec, bool generated, uint32_t n, uint32_t l
     const uint32_t c = (lanes + (uint32_t)sms - 1) / (uint32_t)sms;
     if (lane_prec != 0 && lane_prec != 1 && lane_prec != 4) return -1;   // the other mixed variants: lanes only
     if (generated && lane_prec == 1) return -1;   // f32 lanes are as fast from one zone on (64 zones pulsed: 20.6 against 22.2)
-    if (c <= (generated ? (lane_prec == 4 ? 10u : 8u) : (lane_prec == 4 ? 8u : 11u))) return 2;
+    if (c <= (generated ? (lane_prec == 4 ? 10u : 8u) : lane_prec == 1 ? 11u : 8u)) return 2;
     if (c <= (lane_prec == 4 ? 26u : 16u)) return 1;
     if (generated) return c <= (lane_prec == 4 ? 42u : 78u) ? 0 : -1;
     return lane_prec != 0 || c <= (n > 24 ? 128u : 400u) ? 0 : -1;
