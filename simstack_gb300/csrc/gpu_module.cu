@@ -835,7 +835,7 @@ SGB_API int32_t gpu_kin_autotune(const GpuKinLaunch *launch, uint32_t kind, GpuK
         }
     }
     // kinds 2 and 4: against what the batch size alone would choose, where that is a group kernel (4,096
-    // cells x 1 s: FP64 23.9 ms against 42.5 for the best lane candidate, mixed 14.7 against 20.8)
+    // cells x 1 s: FP64 22.8 ms against 42.5 for the best lane candidate, mixed 14.7 against 20.8)
     bool by_size = false;
     g.tuned[launch->precision] = false;
     const AdvanceShape untuned = shape_for(launch->precision, launch->lane_count ? launch->lane_count : launch->padded, true);

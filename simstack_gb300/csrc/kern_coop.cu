@@ -415,7 +415,7 @@ struct CoopCell {
     // elements make 1/B of the trips to shared memory (FP32) or L2 (FP64). The buffers are the
     // stage vectors K (multipliers) and the four vectors after them (U rows), free until the
     // stages begin, so B is 4 in FP64 and 8 in FP32; the pattern words use x32. Measured on 200 species /
-    // 1,200 reactions, cycles per factorisation: FP64 one CTA per SM 3.05M -> 1.90M, two (per pair of
+    // 1,200 reactions, cycles per factorisation: FP64 one CTA per SM 3.05M -> 1.85M, two (per pair of
     // cells) 2.62M, most of it FP64 instructions at the rate of their unit; FP32 550k -> 357k.
     template <uint32_t B>
     __device__ void factor_panels(Cf ghinv) {
