@@ -563,7 +563,7 @@ SGB_API int32_t gpu_kin_set_mech(const KinMech *mech, const KinMethod *method, c
         if (e != cudaSuccess) return (int32_t)e;
         g.d_coop_image = g.coop_image_buffer;
     }
-    g.plans = true;
+    g.plans = !g.group.starved;
     return 0;
 }
 

@@ -76,10 +76,12 @@ struct GroupSet {
     uint32_t offset[3][3] = {};
     GroupHead head[3][3] = {};
     bool rodas3 = false;
+    bool starved = false;   // the last build found no device memory: worth another
 
     // No kernel may be using the images of the mechanism before.
     cudaError_t build(const KinMech &mech, bool method_rodas3) {
         dev = nullptr;
+        starved = false;
         std::vector<uint32_t> all, one;
         for (int g = 0; g < 3; ++g)
             for (int f = 0; f < 3; ++f) {
@@ -94,6 +96,7 @@ struct GroupSet {
             if (cudaMalloc((void **)&buffer, all.size() * 4) != cudaSuccess) {   // no memory: the lane kernels run alone
                 cudaGetLastError();
                 buffer = nullptr;
+                starved = true;
                 return cudaSuccess;
             }
             capacity = all.size() * 4;
