@@ -790,7 +790,7 @@ struct CoopCell {
     // FP32, a barrier per 32 columns: a warp solves its 32 rows by shuffle (~30 cycles a column; the barriers of
     // eight-column blocks cost more than they spread) from coefficients it loaded once for both
     // directions, the rows past it have theirs on their way meanwhile. No pattern or bounds tests:
-    // off the pattern the LU is zero, and so are the coefficients and x of rows past the end (x has
+    // off the pattern the LU is zero, and so are the triangle and x of rows past the end (x has
     // room for whole blocks). 34k -> 24k cycles per solve of 200 species.
     static __device__ __noinline__ void solve_rows_f32(const Cf *a, uint32_t n, uint32_t ld, float *x, uint32_t threads) {
         constexpr uint32_t B = 32;
@@ -828,7 +828,7 @@ struct CoopCell {
         for (uint32_t q = 0; q < B; ++q) inv = lane == q ? cd[q] : inv;
         float ct[B];        // the own block's triangle, zero elsewhere: a step is a shuffle and an FMA
 #pragma unroll
-        for (uint32_t q = 0; q < B; ++q) ct[q] = lane > q ? cd[q] : 0.0f;
+        for (uint32_t q = 0; q < B; ++q) ct[q] = mine && lane > q ? cd[q] : 0.0f;   // (past the end cd is row 0's)
         sync_rows(threads);   // x is read
         for (uint32_t b = 0; b < blocks; ++b) {
             if (warp == b) {
