@@ -130,6 +130,7 @@ struct CoopCell {
     uint32_t iterations, transitions;
     int phase;
     bool pending, reject_last, reject_more;
+    bool on_pattern;        // mixed: this attempt touches the pattern's elements alone
 
     __device__ __forceinline__ void sync() const { __syncthreads(); }
     __device__ __forceinline__ bool bit(uint32_t i, uint32_t j) const { return (pat[i * 8u + (j >> 5)] >> (j & 31u)) & 1u; }
@@ -315,7 +316,7 @@ struct CoopCell {
     // l(i,k) = a[i][k] * (1/U(k,k)) and stores it once the row is done, so a pivot
     // needs one barrier (FP32) or two (FP64: the shared inverse).
     __device__ void factor(Cf ghinv) {
-        if (n >= kCoopPanelMin && NT >= n) {
+        if (n >= kCoopPanelMin && NT >= n && !(kMixed && on_pattern)) {
             if constexpr (kMixed) factor_panels_f32(ghinv);
             else factor_panels<4>(ghinv);
             return;
@@ -581,7 +582,7 @@ struct CoopCell {
     }
 
     // factor_panels in FP32, B = 8, without pattern tests: an element off the pattern is zero and stays
-    // zero, and a product with it changes no value. The block's rows lie in one warp, which
+    // zero, and a product with it changes no finite value (the others: attempt()). The block's rows lie in one warp, which
     // factors them by shuffle (a reciprocal, one shuffle per entry), so a panel needs two barriers and
     // not one per pivot; trailing rows are walked 64 columns at a time, the multipliers of a row
     // (two 16-byte broadcasts) serving sixteen FMAs per lane. 357k cycles per factorisation of 200
@@ -704,7 +705,7 @@ struct CoopCell {
     // diagonal holding 1/U(k,k)) descending, then the diagonal.
     template <class V>
     __device__ void solve(V *x) {
-        if (NT < n) {
+        if (NT < n || (kMixed && on_pattern)) {
             solve_plain(x);
             return;
         }
@@ -858,7 +859,7 @@ struct CoopCell {
         }
     }
 
-    // In 32-column blocks, for CTAs of fewer threads than rows: a warp solves the diagonal block with
+    // In 32-column blocks, for CTAs of fewer threads than rows and attempts on the pattern alone: a warp solves the diagonal block with
     // shuffles, then every row outside it takes the block's updates.
     template <class V>
     __device__ void solve_plain(V *x) {
@@ -945,8 +946,12 @@ struct CoopCell {
         }
     }
 
-    // One pass of kin_integrate's step loop (kin_solver.h:216-311).
-    __device__ void attempt(const DevArgs &A) {
+    // One pass of kin_integrate's step loop (kin_solver.h:216-311); true: nothing is decided, and it is to be
+    // made again with on_pattern. The mixed path's panels and solves multiply by the zeros off the
+    // pattern, which changes no finite value, but an element of the LU or of a solution past FP32's range
+    // makes NaNs of them, which reach species that it has nothing to do with. Either leaves some
+    // stage value that is not finite.
+    __device__ bool attempt(const DevArgs &A) {
         const double h_min = A.ctl.h_min, rtol = A.ctl.rtol, atol = A.ctl.atol;
         const double inv_n = 1.0 / (double)n;
         double remaining = seg_end - t;
@@ -1009,9 +1014,11 @@ struct CoopCell {
         }
 
         // y_new into ytmp and the weighted RMS error (kin_solver.h:263-280)
+        bool finite = true;
         for (uint32_t s = tid; s < n; s += NT) {
             double ynew = y[s], yerr = 0.0;
             for (int st = 0; st < S; ++st) {
+                if (kMixed) finite = finite && (__double2hiint(K[(size_t)st * n + s]) & 0x7ff00000) != 0x7ff00000;
                 const double mc = M::m(A, st), ec = M::e(A, st);
                 if (mc != 0.0) ynew = sgb_fma(mc, K[(size_t)st * n + s], ynew);
                 if (ec != 0.0) yerr = sgb_fma(ec, K[(size_t)st * n + s], yerr);
@@ -1020,7 +1027,11 @@ struct CoopCell {
             qv[s] = yerr / scale;
             ytmp[s] = ynew;
         }
-        sync();
+        if constexpr (kMixed) {
+            if (__syncthreads_or(!finite) && !on_pattern && NT >= n) return true;
+        } else {
+            sync();
+        }
         if (tid == 0) {   // error norm and step factor once, shared through red[0..1]
             double e = 0.0;
 #pragma unroll 8
@@ -1061,6 +1072,7 @@ struct CoopCell {
         rejects = rejects + (ok ? 0.0 : 1.0);
         if (!(t < seg_end && !(failed > 0.0))) phase = kPhaseSegFinish;
         sync();
+        return false;
     }
 };
 
@@ -1132,7 +1144,8 @@ __global__ void __launch_bounds__(512, 1) kin_coop_kernel(const __grid_constant_
         C.load(A, cell);
         while (C.settle(A, cell)) {
             const long long t_attempt = clock64();
-            C.attempt(A);
+            C.on_pattern = false;
+            while (C.attempt(A)) C.on_pattern = true;
 #ifdef SGB_COOP_PROFILE
             if (threadIdx.x == 0) atomicAdd(&g_coop_phase_cycles[5], (unsigned long long)(clock64() - t_attempt));
 #else
