@@ -239,15 +239,16 @@ SGB_API int32_t gpu_kin_set_refinement(uint32_t sweeps);
 SGB_API int32_t gpu_kin_set_mixed_variant(uint32_t variant);
 /* Straggler hand-off for precision 0 (0 = off; default 600): in one advance, a cell still
  * stepping after `attempts` step attempts on its lane is parked and finished right after by a
- * group kernel (a warp per cell), so a few very stiff cells no longer run alone on single lanes
+ * group kernel (a warp per cell; the cooperative kernel where the mechanism has no schedule
+ * image, kin_mech_group_image), so a few very stiff cells no longer run alone on single lanes
  * at the end of the launch; the results keep the same bits. While it is on, a CTA of the queue
  * kernel (FP64, and the default mixed variant) also parks its last few cells once the queue is dry. */
 SGB_API int32_t gpu_kin_set_straggler_budget(uint32_t attempts);
 /* Per-thread stack (local memory) reservation of the current context: set it when set_bytes
  * is nonzero; *current receives the value in force. */
 SGB_API int32_t gpu_stack_limit(uint64_t set_bytes, uint64_t *current);
-/* Kept for callers (32..256, multiple of 32): parked cells run on the group kernels, which choose their
- * own shape. */
+/* Threads per parked cell (32..256, multiple of 32; default 128) where the cooperative kernel finishes it; the
+ * group kernels choose their own shape. */
 SGB_API int32_t gpu_kin_set_straggler_block(uint32_t threads);
 /* Cells parked by the last advance that used the hand-off (waits for the module stream). */
 SGB_API int32_t gpu_kin_parked_cells(uint32_t *count);

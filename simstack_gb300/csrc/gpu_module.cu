@@ -96,8 +96,10 @@ struct Module {
     cudaEvent_t ev_in[kMaxChunks] = {}, ev_kern[kMaxChunks] = {};
     cudaEvent_t pipe_begin = nullptr, pipe_end = nullptr, pipe_after = nullptr;
     // straggler hand-off: cells past `straggler_budget` step attempts in one launch are parked
-    // and finished by a group kernel on the same stream
+    // and finished by a group kernel on the same stream, or by the cooperative kernel (one CTA per
+    // cell) where the mechanism has no schedule images
     uint32_t straggler_budget = 600;  // FP64 step attempts per launch before a cell is handed on
+    uint32_t straggler_block = 128;   // threads per parked cell of the cooperative kernel
     SuspendRec *d_suspend = nullptr;
     uint32_t *d_suspend_count = nullptr;
     void *d_coop_image = nullptr;     // coop_image_buffer while the mechanism has an image
@@ -117,7 +119,7 @@ constexpr uint32_t kSuspendCap = 1u << 16;       // parked cells per launch
 // different reservations and reallocations); 3,840 bytes covers every default-path kernel of
 // the shipped mechanism (the FP64 lanes need 3,680) and was the fastest such size measured.
 constexpr size_t kStackReserveBytes = 3840;
-constexpr uint32_t kCoopCtasPerSm = 8;           // cooperative CTAs per SM at most (tuning kind 3)
+constexpr uint32_t kCoopCtasPerSm = 8;           // cooperative CTAs per SM at most
 
 
 const GpuKinTuning kDefaultTuning = {2u, 128u, 0u, 0u, 0.0f};   // CTA-synchronous queue, 128 threads, 255 registers
@@ -202,8 +204,12 @@ AdvanceShape shape_for(uint32_t prec, uint32_t lanes, bool with_mode) {
 }
 
 // Whether a lane advance of this precision hands cells on: stragglers (FP64) and the last ones of the
-// CTA queue kernel (FP64 and the default mixed variant).
-bool handoff(uint32_t prec) { return g.straggler_budget && g.group.dev && (lane_prec(prec) == 0 || lane_prec(prec) == 4); }
+// CTA queue kernel (FP64 and the default mixed variant). Without schedule images: stragglers only, to the
+// cooperative kernel.
+bool handoff(uint32_t prec) {
+    if (!g.straggler_budget) return false;
+    return g.group.dev ? lane_prec(prec) == 0 || lane_prec(prec) == 4 : prec == 0 && g.d_coop_image;
+}
 
 // The group kernel on cells of `A` (its cursor is zeroed first), or on the parked ones (A.resume).
 cudaError_t launch_group(uint32_t prec, int group, const DevArgs &A0, cudaStream_t stream) {
@@ -233,8 +239,8 @@ cudaError_t local_bytes(uint32_t prec, const GpuKinTuning &t, size_t *bytes) {
 }
 
 // Launches one advance of `A` in shape `s` on the module stream; the lane kernels with a straggler
-// budget (precision 0) park cells still stepping after that many attempts, and a group kernel
-// finishes them right after, with the same bits.
+// budget (precision 0) park cells still stepping after that many attempts, and a group kernel or the
+// FP64 cooperative kernel finishes them right after, with the same bits.
 cudaError_t launch_advance(uint32_t prec, const AdvanceShape &s, const DevArgs &A0) {
     if (A0.lanes == 0) return cudaSuccess;
     if (s.group >= 0) return launch_group(prec, s.group, A0, g.stream);
@@ -254,7 +260,7 @@ cudaError_t launch_advance(uint32_t prec, const AdvanceShape &s, const DevArgs &
     if (!handoff(prec)) return launch_lanes(prec, t, A0);
     DevArgs A = A0;
     A.budget = prec == 0 ? g.straggler_budget : 0;
-    A.drain = t.kind == 2 ? group_drain(lane_prec(prec), g.generated, t.block) : 0;
+    A.drain = t.kind == 2 && g.group.dev ? group_drain(lane_prec(prec), g.generated, t.block) : 0;
     A.suspend_cap = kSuspendCap;
     A.suspend_count = g.d_suspend_count;
     A.suspend = g.d_suspend;
@@ -263,6 +269,14 @@ cudaError_t launch_advance(uint32_t prec, const AdvanceShape &s, const DevArgs &
     if (e != cudaSuccess) return e;
     A.resume = 1;
     A.cursor = g.d_cursor;
+    if (!g.group.dev) {
+        A.budget = 0;
+        A.tables = g.d_coop_image;
+        A.table_bytes = g.coop_head.bytes;
+        e = cudaMemsetAsync(A.cursor, 0, sizeof(uint32_t), g.stream);
+        if (e != cudaSuccess) return e;
+        return coop_launch(0, A, g.coop_head, g.d_coop_scratch, g.coop_grid, g.straggler_block, g.stream);
+    }
     return launch_group(prec, prec == 0 ? 0 : 1, A, g.stream);   // mixed CTAs park few: 16 lanes per cell
 }
 
@@ -549,7 +563,7 @@ SGB_API int32_t gpu_kin_set_mech(const KinMech *mech, const KinMethod *method, c
     g.plans = false;
     e = g.group.build(*mech, g.group.rodas3);
     if (e != cudaSuccess) return (int32_t)e;
-    // the cooperative image of the same mechanism (tuning kind 3, mode 1)
+    // the cooperative image of the same mechanism (tuning kind 3, mode 1, hand-off without group images)
     // (the buffers are kept while they are large enough: the stream is idle here)
     g.d_coop_image = nullptr;
     std::vector<uint8_t> coop;
@@ -887,7 +901,8 @@ SGB_API int32_t gpu_kin_set_straggler_budget(uint32_t attempts) {
 
 SGB_API int32_t gpu_kin_set_straggler_block(uint32_t threads) {
     if (threads < 32 || threads > 256 || (threads & 31)) return (int32_t)cudaErrorInvalidValue;
-    return 0;   // parked cells run on the group kernels, which choose their own shape
+    g.straggler_block = threads;
+    return 0;
 }
 
 SGB_API int32_t gpu_kin_parked_cells(uint32_t *count) {

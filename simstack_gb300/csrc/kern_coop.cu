@@ -156,6 +156,20 @@ struct CoopCell {
         sync();
     }
 
+    // A parked cell: its scalar state from the record (load() read y, k, src and failed).
+    __device__ void restore(const SuspendRec &r) {
+        t = r.t;
+        h = r.h;
+        seg_end = r.seg_end;
+        applied = r.applied;
+        pending = (r.flags & 1u) != 0;
+        reject_last = (r.flags & 2u) != 0;
+        reject_more = (r.flags & 4u) != 0;
+        iterations = r.iterations;
+        transitions = r.transitions;
+        phase = kPhaseStepping;
+    }
+
     __device__ void store(const DevArgs &A, uint32_t cell) {
         const uint32_t p = A.padded;
         for (uint32_t s = tid; s < n; s += NT) A.y[(size_t)s * p + cell] = y[s];
@@ -1139,9 +1153,17 @@ __global__ void __launch_bounds__(512, 1) kin_coop_kernel(const __grid_constant_
         __syncthreads();
         const uint32_t idx = cell_s;
         __syncthreads();
-        const uint32_t cell = idx;
-        if (cell >= A.lanes) break;
-        C.load(A, cell);
+        uint32_t cell = idx;
+        if (PREC == 0 && A.resume) {   // cells parked by a lane kernel of this launch
+            if (idx >= min(*(volatile uint32_t *)A.suspend_count, A.suspend_cap)) break;
+            const SuspendRec r = A.suspend[idx];
+            cell = r.cell;
+            C.load(A, cell);
+            C.restore(r);
+        } else {
+            if (idx >= A.lanes) break;
+            C.load(A, cell);
+        }
         while (C.settle(A, cell)) {
             const long long t_attempt = clock64();
             C.on_pattern = false;
@@ -1199,7 +1221,8 @@ size_t coop_smem_bytes_for(int prec, const CoopMech &h) { return coop_smem_bytes
 size_t coop_scratch_doubles_for(int prec, const CoopMech &h) { return coop_scratch_doubles(prec, h); }
 
 // The cooperative kernel on `A` (A.tables the coop image, A.cursor zeroed):
-// lanes [0, A.lanes); `scratch` holds grid slots of coop_scratch_doubles_for(prec) doubles.
+// lanes [0, A.lanes), or with A.resume (FP64) the cells a lane kernel parked;
+// `scratch` holds grid slots of coop_scratch_doubles_for(prec) doubles.
 cudaError_t coop_launch(int prec, const DevArgs &A0, const CoopMech &head, double *scratch, uint32_t grid,
                                uint32_t block, cudaStream_t s) {
     void (*fn)(DevArgs, double *, uint64_t) = prec == 0 ? kin_coop_kernel<0> : kin_coop_kernel<2>;

@@ -141,13 +141,13 @@ struct DevArgs {
     uint32_t table_bytes;      // bytes to stage (multiple of 16)
     // straggler hand-off (queue and static kernels, precision 0): a cell that has taken
     // `budget` step attempts in this launch parks its scalar state in `suspend` and leaves; a
-    // group kernel finishes it (0 = never). Group kernels: a warp with such a cell stops claiming.
+    // group kernel (or the cooperative kernel) finishes it (0 = never). Group kernels: a warp with such a cell stops claiming.
     uint32_t budget;
     uint32_t drain;            // CTA queue kernel: a CTA down to this many cells parks them (the queue is dry then)
     uint32_t suspend_cap;
     uint32_t *suspend_count;
     struct SuspendRec *suspend;
-    uint32_t resume;           // group kernel: take cells from the suspension list
+    uint32_t resume;           // group and cooperative kernels: take cells from the suspension list
     uint32_t coop_smem_budget; // cooperative kernel: shared-memory bytes the term lists may fill up to
 };
 

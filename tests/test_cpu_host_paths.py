@@ -10,7 +10,10 @@ from fake_runtime import Fake
 
 @pytest.fixture
 def fake(monkeypatch):
-    return Fake(monkeypatch)
+    f = Fake(monkeypatch)
+    yield f
+    f.module.set_straggler_budget(sg.DEFAULT_STRAGGLER_BUDGET)   # what gpu_init leaves as it is
+    sg.check(sg.lib().gpu_kin_set_straggler_block(128), "gpu_kin_set_straggler_block")
 
 
 def advanced(fake, cells=100, precision=0, **kw):
@@ -29,3 +32,23 @@ def test_images_that_found_no_memory_are_tried_again(fake):
     assert "kin_group_kernel" not in advanced(fake)[0]["name"]
     fake.module.set_mech(km)
     assert "kin_group_kernel" in advanced(fake)[0]["name"]
+
+
+def reordered(km):
+    """The record with two entries of a row's lower list in the other order: valid, but without group images."""
+    km = sg.KinMech.from_buffer_copy(sg.kinmech_bytes(km))
+    i = next(i for i in range(17) if km.lower_begin[i + 1] - km.lower_begin[i] > 1)
+    a, b = km.lower[km.lower_begin[i]], km.lower[km.lower_begin[i] + 1]
+    (a.index, a.col), (b.index, b.col) = (b.index, b.col), (a.index, a.col)
+    return km
+
+
+def test_stragglers_without_group_images_go_to_the_cooperative_kernel(fake):
+    fake.module.set_mech(reordered(sg.Model.air().kinmech()))
+    sg.check(sg.lib().gpu_kin_set_straggler_block(64), "gpu_kin_set_straggler_block")
+    lanes, rest = advanced(fake)
+    assert "kin_queue_cta_kernel" in lanes["name"] and lanes["budget"] > 0 and lanes["drain"] == 0
+    assert "kin_coop_kernel<0>" in rest["name"] and rest["resume"] == 1 and rest["block"] == 64
+    assert len(advanced(fake, precision=2)) == 1   # mixed cells stay on their lanes
+    fake.module.set_straggler_budget(0)
+    assert len(advanced(fake)) == 1
