@@ -561,11 +561,11 @@ SGB_API int32_t gpu_kin_set_mech(const KinMech *mech, const KinMethod *method, c
     g.group.rodas3 = method_is_rodas3(method);
     if (same) return 0;
     g.plans = false;
+    g.d_coop_image = nullptr;   // the record before's, whatever becomes of the images
     e = g.group.build(*mech, g.group.rodas3);
     if (e != cudaSuccess) return (int32_t)e;
     // the cooperative image of the same mechanism (tuning kind 3, mode 1, hand-off without group images)
     // (the buffers are kept while they are large enough: the stream is idle here)
-    g.d_coop_image = nullptr;
     std::vector<uint8_t> coop;
     if (coop_image(*mech, &coop)) {
         memcpy(&g.coop_head, coop.data(), sizeof(CoopMech));

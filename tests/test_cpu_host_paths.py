@@ -52,3 +52,16 @@ def test_stragglers_without_group_images_go_to_the_cooperative_kernel(fake):
     assert len(advanced(fake, precision=2)) == 1   # mixed cells stay on their lanes
     fake.module.set_straggler_budget(0)
     assert len(advanced(fake)) == 1
+
+
+def test_a_failed_set_mech_leaves_no_other_mechanisms_tables(fake):
+    """Images that could not be written: the cooperative shape has nothing to run on and says so."""
+    small = sg.Model.synthetic(seed=2, species=3, reactions=6)
+    fake.module.set_mech(small.kinmech())
+    fake.module.set_tuning(kind=3, block=32)
+    fake.fail("cudaMemcpy", error=999)
+    with pytest.raises(sg.GpuError):
+        fake.module.set_mech(sg.Model.air().kinmech())
+    with pytest.raises(sg.GpuError):
+        fake.module.integrate(sg.air_cells(8, seed=1), 1.0)
+    assert fake.launches() == []
