@@ -250,7 +250,8 @@ SGB_API int32_t gpu_stack_limit(uint64_t set_bytes, uint64_t *current);
 /* Threads per parked cell (32..256, multiple of 32; default 128) where the cooperative kernel finishes it; the
  * group kernels choose their own shape. */
 SGB_API int32_t gpu_kin_set_straggler_block(uint32_t threads);
-/* Cells parked by the last advance that used the hand-off (waits for the module stream). */
+/* Cells parked by the last advance with the hand-off on: none where the batch ran on the group kernels (waits
+ * for the module stream). */
 SGB_API int32_t gpu_kin_parked_cells(uint32_t *count);
 SGB_API uint32_t gpu_kin_get_mixed_variant(void);
 /* Poll limit of the bounded waits with which the table-driven kernels stage a mechanism's

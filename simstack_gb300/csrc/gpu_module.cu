@@ -102,6 +102,7 @@ struct Module {
     uint32_t straggler_block = 128;   // threads per parked cell of the cooperative kernel
     SuspendRec *d_suspend = nullptr;
     uint32_t *d_suspend_count = nullptr;
+    bool parked = false;              // the last advance with the hand-off on left its count there (else: none parked)
     void *d_coop_image = nullptr;     // coop_image_buffer while the mechanism has an image
     void *coop_image_buffer = nullptr;
     size_t coop_image_bytes = 0, coop_scratch_bytes = 0;
@@ -243,7 +244,10 @@ cudaError_t local_bytes(uint32_t prec, const GpuKinTuning &t, size_t *bytes) {
 // FP64 cooperative kernel finishes them right after, with the same bits.
 cudaError_t launch_advance(uint32_t prec, const AdvanceShape &s, const DevArgs &A0) {
     if (A0.lanes == 0) return cudaSuccess;
-    if (s.group >= 0) return launch_group(prec, s.group, A0, g.stream);
+    if (s.group >= 0) {
+        if (handoff(prec)) g.parked = false;
+        return launch_group(prec, s.group, A0, g.stream);
+    }
     const GpuKinTuning &t = s.t;
     if (t.kind == 3) {   // cooperative decomposition: one cell per CTA of t.block threads (32: one warp per cell)
         if (!g.d_coop_image || prec == 1) return cudaErrorInvalidValue;
@@ -264,6 +268,7 @@ cudaError_t launch_advance(uint32_t prec, const AdvanceShape &s, const DevArgs &
     A.suspend_cap = kSuspendCap;
     A.suspend_count = g.d_suspend_count;
     A.suspend = g.d_suspend;
+    g.parked = true;
     cudaError_t e = cudaMemsetAsync(g.d_suspend_count, 0, sizeof(uint32_t), g.stream);
     if (e == cudaSuccess) e = launch_lanes(prec, t, A);
     if (e != cudaSuccess) return e;
@@ -907,6 +912,8 @@ SGB_API int32_t gpu_kin_set_straggler_block(uint32_t threads) {
 
 SGB_API int32_t gpu_kin_parked_cells(uint32_t *count) {
     if (!g.ready || !count) return (int32_t)cudaErrorInvalidValue;
+    *count = 0;
+    if (!g.parked) return (int32_t)cudaStreamSynchronize(g.stream);
     cudaError_t e = cudaMemcpyAsync(count, g.d_suspend_count, sizeof(uint32_t), cudaMemcpyDeviceToHost, g.stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(g.stream);
     return (int32_t)e;

@@ -54,6 +54,10 @@ extern "C" {
 
 // ---- for the tests ----
 void fake_reset_launches() { launches.clear(); }
+void fake_reset_errors() {
+    failing.clear();
+    last = cudaSuccess;
+}
 uint32_t fake_launch_count() { return (uint32_t)launches.size(); }
 const char *fake_launch_name(uint32_t i) { return launches[i].name.c_str(); }
 // grid, block, lanes, resume, budget, drain, wait_polls of launch i, and its tables

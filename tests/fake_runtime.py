@@ -29,7 +29,8 @@ class Fake:
         monkeypatch.setattr(sg, "_lib", None)
         self.L = sg.lib()
         self.L.fake_launch_name.restype = C.c_char_p
-        self.module = sg.Module(0, 1 << 20)
+        self.L.fake_reset_errors()
+        self.module = sg.Module(0, 64 << 20)
         self.L.fake_reset_launches()
 
     def fail(self, call: str, after: int = 0, error: int = 2) -> None:

@@ -65,3 +65,15 @@ def test_a_failed_set_mech_leaves_no_other_mechanisms_tables(fake):
     with pytest.raises(sg.GpuError):
         fake.module.integrate(sg.air_cells(8, seed=1), 1.0)
     assert fake.launches() == []
+
+
+@pytest.mark.parametrize("precision", [0, 2])
+def test_parked_cells_are_the_last_advances(fake, precision):
+    """A batch on the group kernels parks nothing, whatever the batch before it parked."""
+    fake.module.set_mech(sg.Model.air().kinmech())
+    fake.L.fake_park(7)
+    lanes, rest = advanced(fake, cells=20000, precision=precision)
+    assert "kin_queue_cta_kernel" in lanes["name"] and rest["resume"] == 1
+    assert fake.module.parked_cells() == 7
+    assert len(advanced(fake, precision=precision)) == 1
+    assert fake.module.parked_cells() == 0
