@@ -216,7 +216,9 @@ bool handoff(uint32_t prec) {
 cudaError_t launch_group(uint32_t prec, int group, const DevArgs &A0, cudaStream_t stream) {
     DevArgs A = A0;
     A.budget = g.straggler_budget;
-    if (g.generated) A.wait_polls = kSpinLimit;   // the caller's limit is for a table mechanism's staging
+    // the caller's limit is for a table mechanism's staging, before any of a cell's steps: parked cells have taken
+    // some, and a mixed one's state is kept as float pairs until it is done
+    if (g.generated || A.resume) A.wait_polls = kSpinLimit;
     cudaError_t e = cudaMemsetAsync(A.cursor, 0, sizeof(uint32_t), stream);
     if (e != cudaSuccess) return e;
     return g.group.launch(lane_prec(prec), group, A, A.resume ? kSuspendCap : A.lanes, g.sms, stream);

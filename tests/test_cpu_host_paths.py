@@ -77,3 +77,18 @@ def test_parked_cells_are_the_last_advances(fake, precision):
     assert fake.module.parked_cells() == 7
     assert len(advanced(fake, precision=precision)) == 1
     assert fake.module.parked_cells() == 0
+
+
+@pytest.mark.parametrize("precision", [0, 2])
+def test_parked_cells_are_finished_whatever_the_wait_limit(fake, precision):
+    """The limit of the table-staging waits ends the lane kernel before it steps a cell; cells that it parked have been
+    stepped, and are not left half-way."""
+    m = sg.Model.synthetic(seed=5, species=8, reactions=24)
+    fake.module.set_mech(m.kinmech())
+    fake.module.set_tuning(kind=2)
+    fake.launches()
+    sg.check(sg.lib().gpu_kin_set_wait_limit(1), "gpu_kin_set_wait_limit")
+    fake.module.integrate(sg.synthetic_cells(m, 500, seed=1), 1.0, precision=precision)
+    sg.check(sg.lib().gpu_kin_set_wait_limit(1 << 24), "gpu_kin_set_wait_limit")
+    lanes, rest = fake.launches()
+    assert lanes["wait_polls"] == 1 and rest["resume"] == 1 and rest["wait_polls"] > 1 << 20
