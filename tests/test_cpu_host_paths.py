@@ -92,3 +92,58 @@ def test_parked_cells_are_finished_whatever_the_wait_limit(fake, precision):
     sg.check(sg.lib().gpu_kin_set_wait_limit(1 << 24), "gpu_kin_set_wait_limit")
     lanes, rest = fake.launches()
     assert lanes["wait_polls"] == 1 and rest["resume"] == 1 and rest["wait_polls"] > 1 << 20
+
+
+CELLS = 64000   # lanes: past the group kernels' sizes, each CTA parks what it has left
+
+
+@pytest.fixture
+def serving(fake):
+    """A table mechanism of three species (160 bytes a cell) and the budget of one request."""
+    m = sg.Model.synthetic(seed=2, species=3, reactions=6)
+    base = 8 * (3 * 3 + 6 + 8) * CELLS + 8 * 3
+    opened = []
+
+    def run(budget, requests):
+        s = sg.Server(budget)
+        opened.append(s)
+        s.set_mech(m.kinmech())
+        y, k = np.full((3, CELLS), 1e-6), np.repeat(m.k_const[:, None], CELLS, 1)
+        for _ in range(requests):
+            s.submit(y, k, 1, 64, 0.05, mechanism=1)
+        running = s.progress()[0]
+        return s.stats(), running, fake.stream_bytes(), fake.launches()
+
+    run.one = base + 256 + table_bytes(fake)
+    yield run
+    for s in opened:
+        s.close()
+
+
+def table_bytes(fake):
+    """A request's table image: the smallest budget that takes a request of one cell tells it."""
+    s = sg.Server(1 << 30)
+    s.submit(np.full((17, 8), 1e10), np.full((44, 8), 1e-10), 1, 8, 0.05)
+    s.progress()
+    n = s.stats()["in_use_bytes"] - 8 * (3 * 17 + 44 + 8) * 8 - 8 * 17 - 256
+    s.close()
+    fake.launches()
+    return n
+
+
+def test_served_hand_off_is_inside_the_budget(serving):
+    stats, running, (now, peak), launches = serving(1 << 30, 1)
+    assert running == 1 and any(k["resume"] for k in launches)
+    assert now <= stats["in_use_bytes"] and peak <= stats["peak_bytes"]
+
+
+def test_served_request_that_fills_the_budget_keeps_its_cells(serving):
+    stats, running, (now, _), launches = serving(serving.one, 1)
+    assert running == 1 and not any(k["resume"] for k in launches)
+    assert now == stats["in_use_bytes"] == serving.one
+
+
+@pytest.mark.parametrize("spare", [0, 100000])
+def test_served_hand_off_keeps_no_request_waiting(serving, spare):
+    stats, running, (now, _), _ = serving(2 * serving.one + spare, 2)
+    assert running == 2 and now <= stats["in_use_bytes"] <= stats["budget_bytes"]
