@@ -482,10 +482,13 @@ SGB_API int32_t gpu_serve_set_mech(const KinMech *mech, const KinMethod *method)
     if (!E.open || !mech || !method) return (int32_t)cudaErrorInvalidValue;
     if (!mech_tables_valid(mech, method)) return (int32_t)cudaErrorInvalidValue;
     if (!E.running.empty() || !E.waiting.empty()) return (int32_t)cudaErrorNotReady;   // requests hold the old tables
+    const cudaError_t e = E.group[1].build(*mech, method_is_rodas3(method));
+    if (e != cudaSuccess) {   // the mechanism before stays, on the lane kernels
+        cudaGetLastError();
+        return (int32_t)e;
+    }
     E.table_mech = *mech;
     E.table_method = *method;
-    const cudaError_t e = E.group[1].build(*mech, method_is_rodas3(method));
-    if (e != cudaSuccess) return (int32_t)e;
     E.have_table_mech = true;
     return 0;
 }

@@ -147,3 +147,21 @@ def test_served_request_that_fills_the_budget_keeps_its_cells(serving):
 def test_served_hand_off_keeps_no_request_waiting(serving, spare):
     stats, running, (now, _), _ = serving(2 * serving.one + spare, 2)
     assert running == 2 and now <= stats["in_use_bytes"] <= stats["budget_bytes"]
+
+
+def test_a_failed_serve_set_mech_keeps_the_mechanism_before(fake):
+    """A request's arrays are read by the species and reactions of the mechanism that is in force."""
+    old, new = sg.Model.synthetic(seed=2, species=3, reactions=6), sg.Model.synthetic(seed=7, species=8, reactions=24)
+    y, k = np.full((3, 8), 1e-6), np.repeat(old.k_const[:, None], 8, 1)
+    with sg.Server(1 << 30) as s:
+        s.set_mech(old.kinmech())
+        s.submit(y, k, 1, 8, 0.05, mechanism=1)
+        s.progress()
+        one = s.stats()["in_use_bytes"]
+        s.drain()
+        fake.fail("cudaMemcpy", error=999)
+        with pytest.raises(sg.GpuError):
+            s.set_mech(new.kinmech())
+        rid = s.submit(y, k, 1, 8, 0.05, mechanism=1)
+        s.progress()
+        assert s.poll(rid)["state"] == "running" and s.stats()["in_use_bytes"] == one
