@@ -182,13 +182,15 @@ struct AdvanceShape {
 };
 
 // The lane kernels' shape for the shipped mechanism, from one GB300 (ms):
-//   f32: one cell per lane to completion, 64 threads per CTA: the queue kernels' votes and barriers cost
-//     more than the refilling gives (pulsed zones, static / CTA queue: 64 zones 20.6 / 32.3, 4,096 zones
-//     20.8 / 33.0, 65,536 zones 21.0 / 22.0)
+//   f32: one cell per lane to completion, 64 threads per CTA, while all cells are on the GPU at once (four
+//     such CTAs per SM): there is nothing to refill, and the queue kernels' votes and barriers cost a half more.
+//     Past that the static kernel waits for the longest cell of every wave (cells per SM, static / CTA
+//     queue: pulsed zones 32 9.7 / 15.2, 128 15.2 / 15.7, 256 26.1 / 28.3, 300 40.0 / 36.7; air cells under a source over
+//     three decades 32 16.0 / 27.8, 128 24.7 / 28.0, 256 48.3 / 51.0, 300 74.9 / 54.1, 2,632 479 / 286)
 //   mixed: once one 128-lane CTA per SM is full, one CTA of 256, whose eight warps fetch the step code
 //     together (128 x 2 / 256 threads: 16,384 cells 26.7 / 32.2, 32,768 41.5 / 33.0, 262,144 228 / 143)
 void lane_rule(uint32_t lp, uint32_t lanes, GpuKinTuning *t) {
-    if (lp == 1) *t = GpuKinTuning{0u, 64u, 0u, 0u, 0.0f};
+    if (lp == 1 && lanes <= 256u * (uint32_t)g.sms) *t = GpuKinTuning{0u, 64u, 0u, 0u, 0.0f};
     if (lp == 4 && lanes > 128u * (uint32_t)g.sms) *t = GpuKinTuning{2u, 256u, 0u, 2u, 0.0f};
 }
 

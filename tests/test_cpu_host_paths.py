@@ -34,6 +34,13 @@ def test_images_that_found_no_memory_are_tried_again(fake):
     assert "kin_group_kernel" in advanced(fake)[0]["name"]
 
 
+def test_f32_lanes_past_one_wave_run_the_queue(fake):
+    """The static kernel does not refill a lane whose cell is done: it takes batches whose cells are all on the GPU."""
+    fake.module.set_mech(sg.Model.air().kinmech())
+    for cells, kernel in ((64, "kin_static_kernel"), (152 * 256, "kin_static_kernel"), (152 * 256 + 8, "kin_queue_cta_kernel")):
+        assert [kernel in k["name"] for k in advanced(fake, cells=cells, precision=1)] == [True], cells
+
+
 def reordered(km):
     """The record with two entries of a row's lower list in the other order: valid, but without group images."""
     km = sg.KinMech.from_buffer_copy(sg.kinmech_bytes(km))
