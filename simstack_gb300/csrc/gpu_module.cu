@@ -268,7 +268,7 @@ cudaError_t launch_advance(uint32_t prec, const AdvanceShape &s, const DevArgs &
     if (!handoff(prec)) return launch_lanes(prec, t, A0);
     DevArgs A = A0;
     A.budget = prec == 0 ? g.straggler_budget : 0;
-    A.drain = t.kind == 2 && g.group.dev ? group_drain(lane_prec(prec), g.generated, t.block) : 0;
+    A.drain = t.kind == 2 && g.group.dev ? group_drain(lane_prec(prec), g.generated, g.mech.species_count, t.block) : 0;
     A.suspend_cap = kSuspendCap;
     A.suspend_count = g.d_suspend_count;
     A.suspend = g.d_suspend;

@@ -44,26 +44,48 @@ constexpr uint32_t kGroupLanes[3] = {8, 16, 32};
 // (in CTAs of four warps; launch() below now takes FP64's shape by the share, which moves 16 lanes forward:)
 //   table FP64, 0.05 s, 1,230 cells (9 per SM), 32 / 16 lanes: 16 species 14.2 / 11.4, 24 species
 //                    19.7 / 17.3, 32 species (0.02 s) 26.7 / 22.9; 1,660 cells 15.6 / 11.9, 20.8 / 17.8, 28.8 / 24.7
-// The table-driven lane kernels keep a cell's arrays in local memory (~1 ms per attempt) and win only
-// where they fill the GPU several times over (0.1 s, 65,536 cells, 8 lanes / lane kernel): FP64 8 species
-// 54 / 51, 16 species 176 / 203, 24 species 513 / 576, 32 species 16,384 cells 339 / 372 and 65,536
-// cells 1,287 / 929 (its cells leave room for three warps per SM); mixed 38 / 50, 118 / 239, 445 / 688.
+// How far table mechanisms go is group_most's.
+inline uint32_t group_most(uint32_t lane_prec, uint32_t n);
 inline int group_rule(uint32_t lane_prec, bool generated, uint32_t n, uint32_t lanes, int sms) {
     const uint32_t c = (lanes + (uint32_t)sms - 1) / (uint32_t)sms;
     if (lane_prec != 0 && lane_prec != 1 && lane_prec != 4) return -1;   // the other mixed variants: lanes only
+    if (!generated && c > group_most(lane_prec, n)) return -1;
     if (generated && lane_prec == 1) return -1;   // f32 lanes are as fast from one zone on (64 zones pulsed: 20.6 against 22.2)
     if (c <= (generated ? (lane_prec == 4 ? 10u : 8u) : lane_prec == 1 ? 11u : 8u)) return 2;
     if (c <= (lane_prec == 4 ? 26u : 16u)) return 1;
-    if (generated) return c <= (lane_prec == 4 ? 42u : 78u) ? 0 : -1;
-    return lane_prec != 0 || c <= (n > 24 ? 128u : 400u) ? 0 : -1;
+    return !generated || c <= (lane_prec == 4 ? 42u : 78u) ? 0 : -1;
+}
+
+// Cells per SM of a table mechanism of n species up to which the group kernels take it. The table-driven lane
+// kernels keep a cell's arrays in local memory, so the larger the mechanism the longer they lose (24
+// species: 1 ms per attempt), but a few species' arrays stay in the caches, and a group of 8 lanes has no
+// work for most of them. Each line is the least over seeded mechanisms of n to 5 n reactions, from the time of
+// 8-lane groups over that of the lanes without a hand-off (0.01 s, at most 120 attempts):
+//   FP64   1 species 16 cells per SM 0.79, 30 1.05; 3: 52 1.02, 98 1.55; 6: 90 0.93, 120 1.14; 8: 120 0.98, 197 1.15;
+//          12: 197 0.96, 300 1.11; 14: 300 0.93, 431 1.05; 16: 300 0.69, 431 0.85; 21: 300 1.01, 430 1.31; 24: 300 0.73, 431 0.88;
+//          32: 140 0.65, 300 1.16
+//   f32    1: 30 0.77, 60 1.37; 2: 60 0.93, 100 1.70; 3: 150 0.75, 197 1.19; 4: 250 0.98, 400 1.11; 6: 400 0.94, 700 1.20; 8: 700 0.94,
+//          1,500 1.21; 10: 1,500 0.90, 3,000 1.07; 12: 2,631 0.59; 24: 1,973 0.53
+//   mixed  1: 50 0.76, 100 1.44; 2: 50 0.58, 100 1.10; 3: 197 0.92, 300 1.08; 4: 500 0.94, 900 1.07; 5: 900 0.89, 2,000 1.13; 6: 2,000 0.92;
+//          7: 2,000 0.80; 16: 986 0.37
+inline uint32_t group_most(uint32_t lane_prec, uint32_t n) {
+    static const uint16_t f32[11] = {0, 30, 60, 150, 250, 400, 400, 600, 750, 1400, 2500};
+    static const uint16_t mixed[7] = {0, 50, 80, 230, 500, 900, 2000};
+    constexpr uint32_t kAll = 0xffffffffu;
+    if (lane_prec == 1) return n < 11 ? f32[n] : kAll;
+    if (lane_prec == 4) return n < 7 ? mixed[n] : kAll;
+    return n <= 9 ? 14 * n : n <= 12 ? 180u : n <= 14 ? 300u : n <= 17 ? 400u : n <= 24 ? 300u : 128u;
 }
 
 // Cells at which a CTA of `block` lanes of the queue kernel parks what it has left: where its attempt costs
 // what a group kernel takes for as many cells at full throughput. Shipped mechanism, cycles: FP64 lanes
 // 308k per 128-lane attempt against ~9.3k per cell and attempt of 8-lane groups (33 cells), mixed
-// 149k per 256 lanes against ~6.5k (23); the table lanes take ~2M per 128, so any CTA that is not full parks.
-inline uint32_t group_drain(uint32_t lane_prec, bool generated, uint32_t block) {
-    if (!generated) return block - 1;
+// 149k per 256 lanes against ~6.5k (23). Table mechanisms, time over that without parking, CTAs of 128 that
+// park from 16 / 127 cells on: FP64 3 species 431 cells per SM 1.00 / 2.07, 986 1.04 / 1.39; 8: 431 1.00 / 1.42; 24: 431 1.00 / 1.03,
+// so they park none; mixed 2: 431 0.93 / 1.64, 986 0.88 / 1.51; 4: 986 0.95 / 1.28; 8: 431 1.00 / 1.07; 10: 431 1.00 / 0.92;
+// 16: 300 1.00 / 0.83. (One species: the launch behind them costs more.)
+inline uint32_t group_drain(uint32_t lane_prec, bool generated, uint32_t n, uint32_t block) {
+    if (!generated) return lane_prec == 0 || n < 2 ? 0u : n < 10 ? block / 8 : block - 1;
     return lane_prec == 0 ? block / 4 : block / 11;
 }
 

@@ -352,16 +352,16 @@ cudaError_t admit(Request *r) {
     sh.grid = resident < needed ? resident : needed;
 
     // The lane kernel's CTAs park their last cells for a group kernel behind it (group_drain), as in a plain
-    // advance: at most grid * drain records (shipped mechanism: half a megabyte; table: nearly every cell of a
-    // request that just fills the GPU, 2 MB). They count against the budget and are done without where it
+    // advance: at most grid * drain records (shipped mechanism: half a megabyte; table, mixed: nearly
+    // every cell of a request that just fills the GPU, 2 MB). They count against the budget and are done without where it
     // has no room for them, or would have none for the next request because of them.
     DevArgs resume = A;
     int resume_group = -1;
-    const uint32_t drain = group_drain(kp, r->generated, sh.block), most = sh.grid * drain;
+    const uint32_t drain = group_drain(kp, r->generated, r->n, sh.block), most = sh.grid * drain;
     const uint32_t cap = most < q.cells ? most : q.cells;
     const uint64_t records = cap * sizeof(SuspendRec), next = E.waiting.empty() ? 0 : E.waiting.front()->footprint;
     const bool room = E.in_use + records + (E.in_use + next <= E.budget ? next : 0) <= E.budget;
-    if (group < 0 && gs.dev && (kp == 0 || kp == 4) && room) {
+    if (group < 0 && gs.dev && (kp == 0 || kp == 4) && drain && room) {
         if (cudaMallocAsync((void **)&r->d_suspend, records, r->stream) == cudaSuccess) {
             r->footprint += records;
             E.in_use += records;

@@ -30,7 +30,7 @@ class Fake:
         self.L = sg.lib()
         self.L.fake_launch_name.restype = C.c_char_p
         self.L.fake_reset_errors()
-        self.module = sg.Module(0, 64 << 20)
+        self.module = sg.Module(0, 256 << 20)
         self.L.fake_reset_launches()
 
     def fail(self, call: str, after: int = 0, error: int = 2) -> None:

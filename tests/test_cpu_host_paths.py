@@ -41,6 +41,28 @@ def test_f32_lanes_past_one_wave_run_the_queue(fake):
         assert [kernel in k["name"] for k in advanced(fake, cells=cells, precision=1)] == [True], cells
 
 
+@pytest.mark.parametrize("precision,species,per_sm,group,drain", [
+    (0, 3, 40, True, 0), (0, 3, 100, False, 0), (0, 8, 110, True, 0), (0, 8, 197, False, 0), (0, 16, 390, True, 0), (0, 16, 431, False, 0),
+    (1, 1, 20, True, 0), (1, 3, 145, True, 0), (1, 3, 431, False, 0), (1, 6, 990, False, 0), (1, 16, 990, True, 0),
+    (2, 1, 98, False, 0), (2, 2, 70, True, 0), (2, 2, 197, False, 16), (2, 3, 431, False, 16), (2, 8, 990, True, 0)])
+def test_table_mechanisms_go_where_they_are_faster(fake, precision, species, per_sm, group, drain):
+    """A few species' lanes beat the groups from far smaller batches on, and a CTA of them parks few of its cells."""
+    if species > 1:
+        m = sg.Model.synthetic(seed=5, species=species, reactions=2 * species)
+    else:
+        m = sg.Model.new()
+        m.add_species("S0", True)
+        m.add_reaction("S0 -> S0 + S0")
+        m.finalize()
+        m.k_const = np.array([0.7])
+    fake.module.set_mech(m.kinmech())
+    fake.launches()
+    fake.module.integrate(sg.synthetic_cells(m, 152 * per_sm, seed=1), 1.0, precision=precision)
+    first, *rest = fake.launches()
+    assert ("kin_group_kernel" in first["name"]) == group and first["drain"] == drain
+    assert len(rest) == (0 if group or precision == 1 else 1)   # the hand-off's
+
+
 def reordered(km):
     """The record with two entries of a row's lower list in the other order: valid, but without group images."""
     km = sg.KinMech.from_buffer_copy(sg.kinmech_bytes(km))
@@ -106,7 +128,7 @@ CELLS = 64000   # lanes: past the group kernels' sizes, each CTA parks what it h
 
 @pytest.fixture
 def serving(fake):
-    """A table mechanism of three species (160 bytes a cell) and the budget of one request."""
+    """A table mechanism of three species (184 bytes a cell), mixed, and the budget of one request."""
     m = sg.Model.synthetic(seed=2, species=3, reactions=6)
     base = 8 * (3 * 3 + 6 + 8) * CELLS + 8 * 3
     opened = []
@@ -117,7 +139,7 @@ def serving(fake):
         s.set_mech(m.kinmech())
         y, k = np.full((3, CELLS), 1e-6), np.repeat(m.k_const[:, None], CELLS, 1)
         for _ in range(requests):
-            s.submit(y, k, 1, 64, 0.05, mechanism=1)
+            s.submit(y, k, 1, 64, 0.05, mechanism=1, precision=2)
         running = s.progress()[0]
         return s.stats(), running, fake.stream_bytes(), fake.launches()
 
