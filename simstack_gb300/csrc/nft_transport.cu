@@ -19,7 +19,7 @@
 // while one warp holds the channel. It is bound by its own instruction issue (~30 per cell
 // and ~56 per site and substep). nft_transport_kernel keeps the state in global memory (L1)
 // and one CTA per group, the boundary values in shared memory with one barrier per substep:
-// longer channels, and runs whose site slots do not fit. 512 channels x 240 cells x 253
+// longer channels, windows of few substeps (resident_pays), and runs whose site slots do not fit. 512 channels x 240 cells x 253
 // substeps: 990 us through memory (3.9 us per substep: load latency and the barrier), 184 us
 // resident (0.73 us).
 //
@@ -428,6 +428,16 @@ bool resident_shape(const GpuNftTransport &t, uint32_t sms, Resident *best) {
     return best->run != 0;
 }
 
+// Whether a window has substeps enough for what the resident kernel does around them: it loads and stores the
+// whole state by single floats a group's row apart, and one lane after the other sums the evaporation,
+// before the old kernel's first substep is through (us resident / through memory, sites every 3): 100 cells in 16
+// groups, 4 substeps 18 / 16, 16 21 / 37; 240 in 64, 4 49 / 28, 12 53 / 57, 24 57 / 104; 500 in 1, 1 24 / 28; 1,000 in 200,
+// 4 410 / 370, 8 445 / 545; 2,304 in 200, 4 980 / 802, 8 1,040 / 1,234. One cell in 200 groups: 60 20.1 / 19.2.
+bool resident_pays(const GpuNftTransport &t) {
+    if (t.groups >= 32) return t.cells > 1 && t.substeps >= (t.cells < 200 ? 32u : t.cells < 1200 ? 24u : 12u);
+    return t.substeps >= (t.cells < 200 ? 16u : t.cells < 400 ? 6u : t.cells < 1000 ? 3u : 1u);
+}
+
 template <bool kFtz> void (*resident_kernel(uint32_t run))(GpuNftTransport, uint32_t, uint32_t) {
     switch (run) {
         case 2: return nft_resident_kernel<kFtz, 2>;
@@ -459,7 +469,7 @@ SGB_API int32_t gpu_nft_transport(const GpuNftTransport *t, float *kernel_ms) {
     if (q == cudaSuccess) q = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (q != cudaSuccess) return (int32_t)q;
     Resident r;
-    if (t->groups <= 0x0fffffffu && resident_shape(*t, (uint32_t)sms, &r)) {   // the channel count fits the grid
+    if (t->groups <= 0x0fffffffu && resident_pays(*t) && resident_shape(*t, (uint32_t)sms, &r)) {   // the channel count fits the grid
         auto kernel = t->flush_denormals ? resident_kernel<true>(r.run) : resident_kernel<false>(r.run);
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r.smem);
         if (e == cudaSuccess) e = module_mark_start();

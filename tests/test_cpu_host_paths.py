@@ -63,6 +63,19 @@ def test_table_mechanisms_go_where_they_are_faster(fake, precision, species, per
     assert len(rest) == (0 if group or precision == 1 else 1)   # the hand-off's
 
 
+@pytest.mark.parametrize("groups,cells,substeps,resident", [
+    (200, 240, 1, False), (200, 240, 23, False), (200, 240, 24, True), (64, 100, 31, False), (64, 100, 32, True), (64, 2304, 11, False),
+    (64, 2304, 12, True), (200, 1, 253, False), (1, 100, 15, False), (1, 100, 16, True), (1, 240, 6, True), (1, 999, 2, False),
+    (1, 999, 3, True), (1, 1000, 0, False), (1, 1000, 1, True), (64, 240, 253, True), (1, 2305, 253, False)])
+def test_film_windows_of_few_substeps_run_through_memory(fake, groups, cells, substeps, resident):
+    """The resident kernel's loads, stores and evaporation sum want some substeps to pay for them."""
+    sites = cells // 3
+    nt = sg.NftTransport(fake.module, groups, cells, sites, 1, 3)
+    nt.run(np.ones(9), 24.0, 150.0, 900.0, 140.0, substeps)
+    (k,) = fake.launches()
+    assert ("nft_resident_kernel" in k["name"]) == resident
+
+
 def reordered(km):
     """The record with two entries of a row's lower list in the other order: valid, but without group images."""
     km = sg.KinMech.from_buffer_copy(sg.kinmech_bytes(km))
