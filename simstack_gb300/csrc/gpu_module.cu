@@ -197,12 +197,13 @@ void lane_rule(uint32_t lp, uint32_t lanes, GpuKinTuning *t) {
 // The shape of an advance of `lanes` cells: the caller's tuning where one was set or measured,
 // else by size. A lane kernel takes as long for one cell per SM as for a full warp of them (shipped
 // mechanism, 1 s: FP64 59 ms, mixed 25 ms up to 16,384 cells), so small batches go to the group
-// kernels (group_rule in group.h).
-AdvanceShape shape_for(uint32_t prec, uint32_t lanes, bool with_mode) {
+// kernels (group_rule in group.h). launch: the cells that a lane kernel has on the GPU at once (the whole batch, if
+// it is not advanced in chunks).
+AdvanceShape shape_for(uint32_t prec, uint32_t lanes, bool with_mode, uint32_t launch = 0) {
     AdvanceShape s = {-1, with_mode ? tuning_for(prec) : g.tuning[prec]};
     if (g.tuned[prec] || (with_mode && g.mode == 1) || s.t.kind == 3) return s;
     if (g.group.dev) s.group = group_rule(lane_prec(prec), g.generated, g.mech.species_count, lanes, g.sms);
-    if (s.group < 0 && g.generated) lane_rule(lane_prec(prec), lanes, &s.t);
+    if (s.group < 0 && g.generated) lane_rule(lane_prec(prec), launch ? launch : lanes, &s.t);
     return s;
 }
 
@@ -699,7 +700,10 @@ SGB_API int32_t gpu_kin_advance_pipelined(const GpuKinLaunch *launch, void *host
         Lc.lane_count = (uint32_t)count;
         DevArgs A;
         fill_args(&Lc, &A);
-        const AdvanceShape shape = shape_for(launch->precision, serial ? A.lanes : (uint32_t)lanes, false);
+        // Lane shapes: mixed by the chunk, as chunks from pageable memory follow one another (50,000 cells in four of
+        // them: 93 ms by the chunk, 110 by the batch); f32 by the two chunks that may run side by side.
+        const uint32_t at_once = launch->precision == 1 ? 2u * A.lanes : A.lanes;
+        const AdvanceShape shape = shape_for(launch->precision, serial ? A.lanes : (uint32_t)lanes, false, at_once);
         if (serial) {
             e = launch_advance(launch->precision, shape, A);
         } else {

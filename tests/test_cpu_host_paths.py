@@ -63,6 +63,19 @@ def test_table_mechanisms_go_where_they_are_faster(fake, precision, species, per
     assert len(rest) == (0 if group or precision == 1 else 1)   # the hand-off's
 
 
+@pytest.mark.parametrize("precision,cells,chunks,kernel,block", [
+    (2, 50000, 4, "kin_queue_cta_kernel", 128), (2, 50000, 2, "kin_queue_cta_kernel", 256), (2, 50000, 1, "kin_queue_cta_kernel", 256),
+    (2, 6000, 4, "kin_group_kernel", None), (1, 50000, 4, "kin_static_kernel", 64), (1, 50000, 2, "kin_queue_cta_kernel", 128)])
+def test_pipelined_chunks_take_a_chunks_shape(fake, precision, cells, chunks, kernel, block):
+    """What a lane kernel has to do is its chunk, not the batch."""
+    fake.module.set_mech(sg.Model.air().kinmech())
+    fake.launches()
+    fake.module.integrate_pipelined(sg.air_cells(cells, seed=1), 1.0, precision=precision, chunks=chunks)
+    launched = fake.launches()
+    assert len(launched) == chunks
+    assert all(kernel in k["name"] and (block is None or k["block"] == block) for k in launched)
+
+
 @pytest.mark.parametrize("groups,cells,substeps,resident", [
     (200, 240, 1, False), (200, 240, 23, False), (200, 240, 24, True), (64, 100, 31, False), (64, 100, 32, True), (64, 2304, 11, False),
     (64, 2304, 12, True), (200, 1, 253, False), (1, 100, 15, False), (1, 100, 16, True), (1, 240, 6, True), (1, 999, 2, False),
