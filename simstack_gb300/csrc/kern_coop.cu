@@ -719,7 +719,10 @@ struct CoopCell {
     // diagonal holding 1/U(k,k)) descending, then the diagonal.
     template <class V>
     __device__ void solve(V *x) {
-        if (NT < n || (kMixed && on_pattern)) {
+        // Few species: the FP32 solve of whole blocks costs more than the elements that there are (a step, by
+        // elements / by blocks, to the solve before both: 3 species 0.95 / 1.29, 8 0.91 / 1.20, 17 0.94 / 1.06, 33 0.91 / 0.98,
+        // 39 0.87 / 0.89).
+        if (NT < n || (kMixed && (on_pattern || n < kCoopPanelMin))) {
             solve_plain(x);
             return;
         }
@@ -873,7 +876,7 @@ struct CoopCell {
         }
     }
 
-    // In 32-column blocks, for CTAs of fewer threads than rows and attempts on the pattern alone: a warp solves the diagonal block with
+    // In 32-column blocks, for CTAs of fewer threads than rows, few mixed species and attempts on the pattern alone: a warp solves the diagonal block with
     // shuffles, then every row outside it takes the block's updates.
     template <class V>
     __device__ void solve_plain(V *x) {
