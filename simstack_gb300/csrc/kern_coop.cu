@@ -73,8 +73,9 @@ __device__ unsigned long long g_coop_phase_cycles[8];
 #endif
 
 // Species from which the elimination runs in panels (a thread per row: CTAs of at least n threads);
-// below, and in smaller CTAs, pivot by pivot.
-constexpr uint32_t kCoopPanelMin = 40;
+// below, and in smaller CTAs, pivot by pivot. FP64 steps with panels, to those with pivots: 6 species 0.96, 17 0.88, 24 0.84,
+// 32 0.80, 39 0.78 (a CTA of a warp: 17 species 0.65, 24 0.51). Mixed steps of 40 species: 0.82.
+constexpr uint32_t kCoopPanelMin = 40, kCoopPanelMinF64 = 4;
 
 // Shared-memory doubles before the mixed path's FP32 arrays.
 __host__ __device__ inline uint32_t coop_smem_doubles(uint32_t n, uint32_t R) { return 11u * n + 2u * R + 8u; }
@@ -330,7 +331,7 @@ struct CoopCell {
     // l(i,k) = a[i][k] * (1/U(k,k)) and stores it once the row is done, so a pivot
     // needs one barrier (FP32) or two (FP64: the shared inverse).
     __device__ void factor(Cf ghinv) {
-        if (n >= kCoopPanelMin && NT >= n && !(kMixed && on_pattern)) {
+        if (n >= (kMixed ? kCoopPanelMin : kCoopPanelMinF64) && NT >= n && !(kMixed && on_pattern)) {
             if constexpr (kMixed) factor_panels_f32(ghinv);
             else factor_panels<4>(ghinv);
             return;
@@ -722,7 +723,7 @@ struct CoopCell {
         // Few species: the FP32 solve of whole blocks costs more than the elements that there are (a step, by
         // elements / by blocks, to the solve before both: 3 species 0.95 / 1.29, 8 0.91 / 1.20, 17 0.94 / 1.06, 33 0.91 / 0.98,
         // 39 0.87 / 0.89).
-        if (NT < n || (kMixed && (on_pattern || n < kCoopPanelMin))) {
+        if (NT < n || (kMixed ? on_pattern || n < kCoopPanelMin : n < kCoopPanelMinF64)) {
             solve_plain(x);
             return;
         }
@@ -876,8 +877,9 @@ struct CoopCell {
         }
     }
 
-    // In 32-column blocks, for CTAs of fewer threads than rows, few mixed species and attempts on the pattern alone: a warp solves the diagonal block with
-    // shuffles, then every row outside it takes the block's updates.
+    // In 32-column blocks, for CTAs of fewer threads than rows, few species and attempts on the pattern
+    // alone: a warp solves the diagonal block with shuffles, then every row outside it takes the block's
+    // updates.
     template <class V>
     __device__ void solve_plain(V *x) {
         const uint32_t nb = (n + 31) / 32;
