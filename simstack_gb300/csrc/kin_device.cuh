@@ -654,7 +654,7 @@ struct LaneDf {
     float khi[R], klo[R], shi[N], slo[N];
     double t, h, seg_end, applied, duration, period, first, count;
     double steps, rejects, pulses, failed;
-    uint32_t iterations, transitions, attempts;
+    uint32_t iterations, transitions;
     int phase;
     bool pending, reject_last, reject_more;
     float lu_r[kLuStride ? 1 : NNZ];
@@ -696,26 +696,7 @@ struct LaneDf {
         t = 0.0;
         applied = 0.0;
         transitions = 0;
-        attempts = 0;
         phase = kPhaseSegStart;
-    }
-
-    // Straggler hand-off (see Lane::park); y goes to the zone block as hi + lo, exact in FP64.
-    __device__ __forceinline__ bool park(const DevArgs &A, uint32_t cell) {
-        const uint32_t slot = atomicAdd(A.suspend_count, 1u);
-        if (slot >= A.suspend_cap) return false;
-        SuspendRec r;
-        r.t = t;
-        r.h = h;
-        r.seg_end = seg_end;
-        r.applied = applied;
-        r.cell = cell;
-        r.iterations = iterations;
-        r.transitions = transitions;
-        r.flags = (pending ? 1u : 0u) | (reject_last ? 2u : 0u) | (reject_more ? 4u : 0u);
-        A.suspend[slot] = r;
-        phase = kPhaseDone;
-        return true;
     }
 
     __device__ __forceinline__ void store(const DevArgs &A, uint32_t i) {
@@ -772,8 +753,6 @@ struct LaneDf {
                 case kPhaseSegStart: seg_start(A); break;
                 case kPhaseSegFinish: seg_finish(A, cell); break;
                 case kPhaseStepping:
-                    if (A.budget && attempts >= A.budget && park(A, cell)) return false;
-                    ++attempts;
                     if (++iterations > A.ctl.max_steps) {
                         failed = 1.0;
                         phase = kPhaseSegFinish;
