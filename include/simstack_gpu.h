@@ -213,7 +213,9 @@ SGB_API int32_t gpu_kin_advance_pipelined(const GpuKinLaunch *launch, void *host
  * at 128 threads, 1: 128 registers, 2: 255 registers at 256 threads, kind 2
  * only; 3: 128 registers at 512 threads, kind 2 only); for kind 3, chunk =
  * CTAs per SM (1..8, 0 = 8). Until one is set or measured, the module chooses by batch
- * size, lane-group kernels (8, 16 or 32 lanes per cell; the same bits) included.
+ * size, lane-group kernels (8, 16 or 32 lanes per cell; the same bits) included;
+ * gpu_kin_get_tuning then answers the default lane shape, not that choice. Once one is set or
+ * measured, batches of every size run it; gpu_init brings the choice by size back.
  * gpu_kin_autotune times the candidates of `kind` on the given launch (which
  * it advances repeatedly on a scratch copy it restores) and keeps the fastest;
  * kind 4 times kinds 2 and 3 together, so the cells-per-warp decomposition is

@@ -34,14 +34,16 @@ constexpr uint32_t kGroupLanes[3] = {8, 16, 32};
 
 // The group shape (index into kGroupLanes) for a batch of `lanes` cells on `sms` SMs, or -1: the lane
 // kernels. Lines in cells per SM, from one advance of 1 s (GB300, 152 SMs; ms for 32 / 16 / 8
-// lanes per cell and the lane kernel):
-//   shipped mechanism  600 cells: FP64 14.0 / 15.4 / 19.6 / 59.4   mixed  9.8 / 10.7 / 14.1 / 24.2
-//                    2,048 cells: FP64 20.9 / 16.7 / 20.1 / 59.4   mixed 12.2 / 11.0 / 14.4 / 25.3
-//                    4,096 cells: FP64 34.2 / 25.8 / 23.2 / 59.5   mixed 18.6 / 16.5 / 16.2 / 25.4
-//                    8,192 cells: FP64 62.7 / 44.3 / 35.4 / 59.4   mixed 33.0 / 26.5 / 23.9 / 24.8
-//                   10,240 cells: FP64 8 lanes 41.7, lane kernel with its hand-off 46.6; 14,336: 52.2, 45.6
-//                    6,144 cells: mixed 8 lanes 21.2, lane kernel with its hand-off 21.9; 7,168: 22.8, 21.7
-// (in CTAs of four warps; launch() below now takes FP64's shape by the share, which moves 16 lanes forward:)
+// lanes per cell and the lane kernel with its hand-off):
+//   shipped mechanism  600 cells: FP64 12.6 / 13.8 / 18.4 / 40.1   mixed  8.8 /  8.9 / 11.7 / 18.9
+//                    1,300 cells: FP64 17.0 / 14.2 / 18.5 / 42.0   mixed  9.4 /  9.0 / 11.9 / 19.7
+//                    2,048 cells: FP64 20.8 / 15.9 / 20.2 / 41.5   mixed 10.9 /  9.9 / 13.0 / 20.0
+//                    2,600 cells: FP64 24.3 / 19.6 / 20.6 / 41.2   mixed 12.2 / 10.8 / 13.1 / 20.1
+//                    4,096 cells: FP64 34.1 / 26.5 / 21.9 / 42.1   mixed 17.1 / 14.9 / 14.4 / 20.9
+//                    6,144 cells: FP64 47.9 / 34.7 / 30.1 / 45.7   mixed 23.3 / 19.5 / 18.8 / 22.3
+//                    7,168 cells: FP64 54.9 / 38.8 / 32.5 / 45.1   mixed 25.7 / 21.2 / 20.6 / 21.6
+//                    8,192 cells: FP64 62.3 / 43.7 / 36.4 / 44.8   mixed 29.9 / 24.7 / 23.0 / 21.7
+//                   11,856 cells: FP64 8 lanes 45.4, lane kernel 46.3; 12,500: 47.0, 46.0
 //   table FP64, 0.05 s, 1,230 cells (9 per SM), 32 / 16 lanes: 16 species 14.2 / 11.4, 24 species
 //                    19.7 / 17.3, 32 species (0.02 s) 26.7 / 22.9; 1,660 cells 15.6 / 11.9, 20.8 / 17.8, 28.8 / 24.7
 // How far table mechanisms go is group_most's.

@@ -9,7 +9,7 @@
 // most of the chip idle for its length. With the cell's work spread over G lanes the same attempt
 // is ~600 (G = 32) to ~1,200 (G = 8, four cells at once) FP64 instructions: the shorter chain where
 // latency counts, at fewer cells per instruction than the lane kernels where throughput does.
-// The rule that chooses between them is in gpu_module.cu (auto_shape).
+// The rule that chooses between them is in group.h (group_rule, group_most).
 //
 // Warps are independent: a warp claims cells from the work queue (or the suspension list) for
 // its 32 / G groups, and its groups take each attempt together. A cell's vectors and dense LU

@@ -395,8 +395,11 @@ struct Resident {
 // that has a site in some lane -- one per stride where the stride divides the run, so that every
 // lane has its sites at the same slots, else every slot -- and the exchange) times 2.5 + 1.75 x
 // (warps per scheduler) cycles, times the waves. Fitted to 240 cells, sites every 3, 253 substeps, us at runs of
-// 2 / 3 / 6 / 9: one group 103 / 101 / 181 / 228, 64 groups 242 / 184 / 237 / 241; it also picks
-// the best of 2..9 measured for 24 to 1,500 cells with strides 1, 3 and 7 to within 15 %.
+// 2 / 3 / 6 / 9: one group 103 / 101 / 181 / 228, 64 groups 242 / 184 / 237 / 241, with the registers that the
+// kernels then took (kRegs; sm_103a, nvcc 13.0, takes 116 115 101 128 255 250 213 243 now, and the choice is as good with
+// either). Over 280 shapes of 24 to 1,500 cells, strides 0, 1, 3, 4 and 7 and 1 to 400 groups its run takes 1.05 times the
+// best run's time on average; 47 of them lie past 1.12 (a run of 2 at a stride of 4, which has its sites in one slot
+// and not in both: 1.2 to 1.4), the worst at 1.73 (400 cells without sites, 100 groups).
 // False: the channel or its site slots do not fit.
 bool resident_shape(const GpuNftTransport &t, uint32_t sms, Resident *best) {
     constexpr uint32_t kRegs[kMaxRun + 1] = {0, 0, 64, 107, 94, 109, 128, 229, 255, 255};
