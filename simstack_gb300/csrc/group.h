@@ -44,6 +44,10 @@ constexpr uint32_t kGroupLanes[3] = {8, 16, 32};
 //                    7,168 cells: FP64 54.9 / 38.8 / 32.5 / 45.1   mixed 25.7 / 21.2 / 20.6 / 21.6
 //                    8,192 cells: FP64 62.3 / 43.7 / 36.4 / 44.8   mixed 29.9 / 24.7 / 23.0 / 21.7
 //                   11,856 cells: FP64 8 lanes 45.4, lane kernel 46.3; 12,500: 47.0, 46.0
+// 8 lanes per cell end where an SM's 64 groups (FP64; mixed 32) are all taken: cells of like numbers of attempts then
+// take a second wave, which only cells that differ fill (averaged zones, one 20 ms step, 8 lanes / the lane kernel: FP64 64 cells
+// per SM 5.1 / 5.1, 68 6.5 / 5.1, 78 7.1 / 5.1; mixed 34 2.2 / 2.2, 36 2.6 / 2.2, 42 2.9 / 2.1; air cells, 0.1 s: FP64 68 36.1 / 40.4,
+// 78 39.8 / 39.8; mixed 36 15.0 / 18.7, 42 16.3 / 18.8).
 //   table FP64, 0.05 s, 1,230 cells (9 per SM), 32 / 16 lanes: 16 species 14.2 / 11.4, 24 species
 //                    19.7 / 17.3, 32 species (0.02 s) 26.7 / 22.9; 1,660 cells 15.6 / 11.9, 20.8 / 17.8, 28.8 / 24.7
 // How far table mechanisms go is group_most's.
@@ -55,7 +59,7 @@ inline int group_rule(uint32_t lane_prec, bool generated, uint32_t n, uint32_t l
     if (generated && lane_prec == 1) return -1;   // f32 lanes are as fast from one zone on (64 zones pulsed: 20.6 against 22.2)
     if (c <= (generated ? (lane_prec == 4 ? 10u : 8u) : lane_prec == 1 ? 11u : 8u)) return 2;
     if (c <= (lane_prec == 4 ? 26u : 16u)) return 1;
-    return !generated || c <= (lane_prec == 4 ? 42u : 78u) ? 0 : -1;
+    return !generated || c <= (lane_prec == 4 ? 34u : 64u) ? 0 : -1;
 }
 
 // Cells per SM of a table mechanism of n species up to which the group kernels take it. The table-driven lane

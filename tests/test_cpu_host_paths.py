@@ -41,6 +41,12 @@ def test_f32_lanes_past_one_wave_run_the_queue(fake):
         assert [kernel in k["name"] for k in advanced(fake, cells=cells, precision=1)] == [True], cells
 
 
+@pytest.mark.parametrize("precision,per_sm,group", [(0, 64, True), (0, 65, False), (2, 34, True), (2, 36, False), (2, 35, False)])
+def test_groups_end_where_they_fill_the_gpu_once(fake, precision, per_sm, group):
+    fake.module.set_mech(sg.Model.air().kinmech())
+    assert ("kin_group_kernel" in advanced(fake, cells=152 * per_sm, precision=precision)[0]["name"]) == group
+
+
 @pytest.mark.parametrize("precision,species,per_sm,group,drain", [
     (0, 3, 40, True, 0), (0, 3, 100, False, 0), (0, 8, 110, True, 0), (0, 8, 197, False, 0), (0, 16, 390, True, 0), (0, 16, 431, False, 0),
     (1, 1, 20, True, 0), (1, 3, 145, True, 0), (1, 3, 431, False, 0), (1, 6, 990, False, 0), (1, 16, 990, True, 0),
@@ -65,7 +71,7 @@ def test_table_mechanisms_go_where_they_are_faster(fake, precision, species, per
 
 @pytest.mark.parametrize("precision,cells,chunks,kernel,block", [
     (2, 50000, 4, "kin_queue_cta_kernel", 128), (2, 50000, 2, "kin_queue_cta_kernel", 256), (2, 50000, 1, "kin_queue_cta_kernel", 256),
-    (2, 6000, 4, "kin_group_kernel", None), (1, 50000, 4, "kin_static_kernel", 64), (1, 50000, 2, "kin_queue_cta_kernel", 128)])
+    (2, 5000, 4, "kin_group_kernel", None), (1, 50000, 4, "kin_static_kernel", 64), (1, 50000, 2, "kin_queue_cta_kernel", 128)])
 def test_pipelined_chunks_take_a_chunks_shape(fake, precision, cells, chunks, kernel, block):
     """What a lane kernel has to do is its chunk, not the batch."""
     fake.module.set_mech(sg.Model.air().kinmech())
